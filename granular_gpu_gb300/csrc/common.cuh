@@ -19,6 +19,7 @@ namespace gg {
 __device__ __forceinline__ float3 f3(float4 a) { return make_float3(a.x, a.y, a.z); }
 __device__ __forceinline__ float3 add3(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ float3 sub3(float3 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }
+__device__ __forceinline__ float3 neg3(float3 a) { return make_float3(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ float3 smul3(float s, float3 a) { return make_float3(s * a.x, s * a.y, s * a.z); }
 __device__ __forceinline__ float3 mul3s(float3 a, float s) { return make_float3(a.x * s, a.y * s, a.z * s); }
 __device__ __forceinline__ float3 div3s(float3 a, float s) { return make_float3(a.x / s, a.y / s, a.z / s); }

@@ -225,6 +225,7 @@ struct gg_system {
   float last_residual_max = 0.0f;     // largest penetration
   int stats_blocks = 0;
   int num_sms = 0;
+  float2* window = nullptr;            // per cell coordinate: the positions whose query cell is within one of it
   int merge_resolve_blocks = 0;  // co-resident blocks of the cooperative merge-schedule kernel
   float nl_skin = 0.0f;                // contact-list skin in use (0 = lists off)
   int64_t steps = 0;
@@ -293,6 +294,7 @@ gg_status reorder_upsampled(gg_system* S, const uint32_t* perm, cudaStream_t st)
 // solve
 gg_status radii_all(gg_system* S, cudaStream_t st);
 gg_status predict(gg_system* S, cudaStream_t st);
+gg_status window_table(gg_system* S, cudaStream_t st);
 gg_status sweep(gg_system* S, int it, cudaStream_t st);
 // last: write the constraint counts (the substep's last sweep, or every
 // sweep of the residual mode); more: another sweep may follow, so record the

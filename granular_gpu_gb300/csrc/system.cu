@@ -216,7 +216,7 @@ static void free_all(gg_system* S) {
                   G.split_slot, G.keep_slot, G.child_pos, G.nl_idx, G.nl_meta, G.nl_acc, G.nl_queue, G.cell_inc, G.ld_sum, G.ld_cnt, G.claim_tgt, G.claimed, G.cell_claim, G.child_cell, G.fdelta, G.pn, S->b.pos, S->b.animated, S->b.pos_alt,
                   S->b.animated_alt, S->b.keys, S->b.perm, S->b.cell_start, S->u.keys, S->u.perm, S->scal,
                   S->stats_partial, S->stage, S->feat, S->xs0, S->warm_target, S->scene_fcap,
-                  S->scene_acc, S->scene_mu};
+                  S->scene_acc, S->scene_mu, S->window};
   for (void* p : ptrs) cudaFree(p);
   if (S->scal_host) cudaFreeHost(S->scal_host);
   sort_scratch_free(S->sort);
@@ -343,6 +343,7 @@ gg_status system_create(const gg_desc* d, gg_system** out) {
   ALLOC(S->b.pos, S->nb); ALLOC(S->b.animated, S->nb); ALLOC(S->b.pos_alt, S->nb);
   ALLOC(S->b.animated_alt, S->nb); ALLOC(S->b.keys, S->nb); ALLOC(S->b.perm, S->nb);
   ALLOC(S->b.cell_start, C1);
+  ALLOC(S->window, std::max(d->cell_size[0], std::max(d->cell_size[1], d->cell_size[2])));
   ALLOC(S->u.keys, S->nu); ALLOC(S->u.perm, S->nu);
   ALLOC(S->scal, 1);
   S->stats_blocks = std::max(1, std::min(4 * S->num_sms, 1024));
@@ -421,6 +422,7 @@ gg_status system_create(const gg_desc* d, gg_system** out) {
   if (S->nu > 0) CHK(cudaMemsetAsync(S->u.vel[S->u.cur], 0, sizeof(float4) * S->nu, st));
 #undef CHK
   // constructor sequence, GranularSystem.cu:54-62
+  if ((rc = window_table(S, st)) != GG_OK) return fail(rc);
   if ((rc = radii_all(S, st)) != GG_OK) return fail(rc);
   if ((rc = boundary_grid(S)) != GG_OK) return fail(rc);
   if ((rc = granular_grid(S)) != GG_OK) return fail(rc);
