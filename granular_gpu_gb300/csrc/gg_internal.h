@@ -49,6 +49,7 @@ struct DevScalars {
   unsigned int disp0_bits;     // max |dt v| of the predict (float bits)
   unsigned int tile_fallback;  // sweep blocks that could not use the shared-memory tile
   int nl_queued[kMaxSweeps];          // per sweep: particles whose contact list is rebuilt
+  int nl_over[kMaxSweeps];     // per sweep: particles with more candidates than a list holds
   unsigned int pen_bits;       // residual mode: largest penetration (float bits)
   unsigned int pen_count;      // residual mode: contacts (particle pairs counted once per side, walls)
   double pen_sum;              // residual mode: sum of their penetrations

@@ -19,8 +19,10 @@
 // nothing, so the sum and its order are unchanged.
 //
 // Kernels.  The default keeps per-particle contact lists across the sweeps
-// of a substep (k_sweep_nlist_build / k_sweep_nlist_keep); without lists,
-// k_sweep_list scans the 27 cells; k_sweep is the pruned one-thread-per-
+// of a substep: a group of lanes to a particle in small systems
+// (k_sweep_group), a thread to a particle in large ones
+// (k_sweep_nlist_build / k_sweep_nlist_keep, with short rebuild queues and
+// overlong lists left to groups); without lists, k_sweep_list scans the 27 cells; k_sweep is the pruned one-thread-per-
 // particle scan the autotuner may pick where lists do not pay.
 #include <algorithm>
 #include <climits>
@@ -53,8 +55,10 @@ struct SweepArgs {
   int4* __restrict__ nl_meta;
   float* __restrict__ nl_acc;
   int32_t* __restrict__ nl_queue;
+  int32_t* __restrict__ nl_over;   // particles with more candidates than a list holds, left to the groups
+  size_t li_row, li_step;          // entry k of particle i's list: nl_idx[i * li_row + k * li_step]
   const uint32_t* __restrict__ cell_inc;
-  int cap;
+  int group_queue;                 // queues up to this length are rebuilt by groups
   float skin;
   float eabs;    // bound on the rounding of one position update
   UDiv div_yz, div_z;  // division by ny * nz and by nz (binning cell of a key)
@@ -442,8 +446,7 @@ __global__ void __launch_bounds__(kWarpThreads) k_sweep_list(SweepArgs a) {
 // of the full scan.  N_u is the sweep's global maximum increment length when
 // that is small enough, else the largest per-cell maximum (recorded by the
 // apply kernel) over the 27 stencil cells and the particle's own cell.
-// Lists whose bound runs out are rebuilt by their own thread; the others are
-// kept.
+// Lists whose bound runs out are rebuilt; the others are kept.
 
 // nl_meta[i].w: the list's length, with a flag when it holds walls; -1 when
 // there were too many candidates to list.
@@ -554,7 +557,7 @@ __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(SweepArgs a) {
       if (m.w & kNlistWalls) target_walls(a, t);
       Sums u;
       const int32_t* __restrict__ li = a.nl_idx + i;
-      apply_entries<MM>(a, t, m.w & kNlistCount, [&](int k) { return __ldcs(li + (size_t)k * a.cap); }, u);
+      apply_entries<MM>(a, t, m.w & kNlistCount, [&](int k) { return __ldcs(li + k * a.li_step); }, u);
       store_sums<MM>(a, i, u);
     } else {
       rebuild = true;
@@ -587,14 +590,14 @@ __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(SweepArgs a) {
 // the queued ones later.
 constexpr int kBuildThreads = 128;
 
-// 8 resident blocks of 128 (64 registers, a few bytes spilled): the queued
-// rebuilds are latency-bound, and the extra warps hide more than the spills
-// cost (72 registers and 7 blocks measured 3 % slower over the sweeps).
+// 8 resident blocks of 128 (64 registers): the rebuilds are latency-bound
+// (72 registers and 7 blocks measured 3 % slower over the sweeps).
 template <int MM>
 __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArgs a, int queued) {
   const Grid& g = a.g;
   const int lane = threadIdx.x & 31;
   const int total = queued ? a.scal->nl_queued[a.it] : a.n;
+  if (queued && total <= a.group_queue) return;  // the groups take a short queue
   for (int base = blockIdx.x * kBuildThreads; base < total; base += gridDim.x * kBuildThreads) {
     const int slot = base + threadIdx.x;
     const bool act = slot < total;
@@ -613,7 +616,7 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArg
     bool walls = false;
     int32_t* __restrict__ li = a.nl_idx + i;
     auto push = [&](int e) {
-      if (cnt < kNlistMax) li[(size_t)cnt * a.cap] = e;
+      if (cnt < kNlistMax) li[cnt * a.li_step] = e;
       ++cnt;
     };
     // candidates in chunks of 32: a mask of those within the reach of the
@@ -666,11 +669,8 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArg
       }
     });
     if (cnt > kNlistMax) {
-      // too many candidates to list: full scan, and again at the next sweep
-      a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, -1);
-      target_walls(a, t);
-      target_masks(a, t);
-      sweep_global<MM>(a, i, t);
+      // too many candidates to list: the groups run them
+      a.nl_over[atomicAdd(&a.scal->nl_over[a.it], 1)] = i;
       continue;
     }
     a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, cnt | (walls ? kNlistWalls : 0));
@@ -678,8 +678,221 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArg
     if (walls) target_walls(a, t);
     Sums u;
     // the list this thread just wrote (its own stores: read back in order)
-    apply_entries<MM>(a, t, cnt, [&](int k) { return li[(size_t)k * a.cap]; }, u);
+    apply_entries<MM>(a, t, cnt, [&](int k) { return li[k * a.li_step]; }, u);
     store_sums<MM>(a, i, u);
+  }
+}
+
+// ------------------------------------------------------------ group sweep
+//
+// The listed sweep with G lanes to a particle, for systems too small to fill
+// the chip with one thread each: a thread alone walks some hundred stencil
+// candidates and a dozen contacts one after the other, and the launch lasts
+// as long as its longest walk, however few particles it rebuilds.  Here the
+// lanes of a group test G candidates at a time, append the hits in order
+// (ballots), run G listed contacts at a time, and add their shares in the
+// reference's order, one lane to a component.  A list that runs out is
+// rebuilt by its own group in the same launch.  Lists are then stored
+// particle by particle.  A particle with more candidates than a list holds
+// runs each full list as the scan goes on, and scans again at the next
+// sweep.
+constexpr int kGroupThreads = 256;
+
+//
+// kQueue: rebuilds the particles of a queue instead: the whole one if it is
+// short, else (the threads have built those lists) the particles whose
+// candidates a list does not hold.
+template <int MM, int G, bool kQueue>
+__global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kGroups = kGroupThreads / G;
+  constexpr int NC = (MM & 2) ? 6 : 3;  // components of a share
+  // a group's rows of shares, padded so that the groups of a warp use
+  // different banks
+  constexpr int kRow = G == 8 ? (NC == 6 ? 56 : 24) : G == 16 ? (NC == 6 ? 112 : 48) : NC * G;
+  constexpr int kStep = 2 * G;  // candidates of a scan step
+  __shared__ int32_t s_list[kGroups][kNlistMax + kStep];
+  __shared__ int4 s_col[kGroups][9];
+  __shared__ float s_share[kGroups][kRow];
+  const Grid& g = a.g;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), grp = threadIdx.x / G;
+  const unsigned glt = (1u << gl) - 1u;
+  auto gballot = [&](bool p) {
+    const unsigned b = __ballot_sync(kAll, p);
+    return G == 32 ? b : (b >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u);
+  };
+  int total = a.n;
+  const int32_t* queue = nullptr;
+  if (kQueue) {
+    const int queued = a.it > 0 ? a.scal->nl_queued[a.it] : INT_MAX;
+    queue = queued <= a.group_queue ? a.nl_queue : a.nl_over;
+    total = queued <= a.group_queue ? queued : a.scal->nl_over[a.it];
+  }
+  for (int base = blockIdx.x * kGroups; base < total; base += gridDim.x * kGroups) {
+  const int slot = base + grp;
+  const bool act = slot < total;
+  // (groups past the end follow along and write nothing)
+  const int is = kQueue ? queue[act ? slot : total - 1] : (act ? slot : total - 1), i = act ? is : -1;
+  Target t;
+  make_target_lite(a, is, a.xs[is], t);
+  int cnt = 0;
+  bool walls = false, rebuild = act;
+  if (!kQueue && a.it > 0) {
+    const int4 m = a.nl_meta[is];
+    const bool same = act && m.w >= 0 && m.x == t.q.x && m.y == t.q.y && m.z == t.q.z;
+    const float A0 = a.nl_acc[is];
+    float A = A0 + nlist_step(a, __uint_as_float(a.scal->inc_norm_bits[a.it - 1]));
+    bool ok = same && nlist_bound_ok(a, A);
+    const bool need = same && !ok;
+    if (__any_sync(kAll, need)) {
+      const float A2 = A0 + nlist_step(a, nlist_cell_bound(a, t.q, a.keys[is]));
+      if (need && nlist_bound_ok(a, A2)) {
+        ok = true;
+        A = A2;
+      }
+    }
+    if (ok) {  // the list is still exact
+      rebuild = false;
+      cnt = m.w & kNlistCount;
+      walls = (m.w & kNlistWalls) != 0;
+      if (gl == 0) a.nl_acc[i] = A;
+    }
+  }
+  if (rebuild) {
+    // the stencil columns, as for_each_stencil_column gives them: their
+    // particles, and the first cell of a column that holds walls
+    const long long zl = max((long long)t.q.z - 1, 0LL), zh = min((long long)t.q.z + 1, (long long)g.nz - 1);
+    for (int k = gl; k < 9; k += G) {
+      int4 col = make_int4(0, 0, -1, 0);
+      const long long x = (long long)t.q.x + k / 3 - 1, y = (long long)t.q.y + k % 3 - 1;
+      if (zl <= zh && x >= 0 && x < g.nx && y >= 0 && y < g.ny) {
+        const int k0 = (int)((x * g.ny + y) * g.nz + zl), nc = (int)(zh - zl + 1);
+        col = make_int4(a.cs[k0], a.cs[k0 + nc], a.bcs[k0] < a.bcs[k0 + nc] ? k0 : -1, nc);
+      }
+      s_col[grp][k] = col;
+    }
+  }
+  __syncwarp();
+  const float Bs = t.Bf + a.skin, Bs2 = Bs * Bs * 1.0001f;
+  const float rcs = t.rc + a.skin;
+  int32_t* row = a.nl_idx + is * a.li_row;
+  bool over = false;
+  float sum = 0.0f;  // component gl of the corrections
+  int c = 0, s_loc = 0;
+  // the scan's place (the same for all groups of a warp): column and cell,
+  // and this lane's candidate there
+  int seg = __any_sync(kAll, rebuild) ? 0 : 27, v = gl;
+  for (;;) {
+    while (seg < 27) {
+      const int k = seg / 3, z = seg - 3 * k;
+      const int4 col = rebuild ? s_col[grp][k] : make_int4(0, 0, -1, 0);
+      const bool cells = __any_sync(kAll, col.z >= 0);  // some group goes cell by cell, walls first
+      int j0 = col.x, np = z == 0 ? col.y - col.x : 0, b0 = 0, nb = 0;
+      if (col.z >= 0) {
+        const bool in = z < col.w;
+        j0 = in ? a.cs[col.z + z] : 0;
+        np = in ? a.cs[col.z + z + 1] - j0 : 0;
+        b0 = in ? a.bcs[col.z + z] : 0;
+        nb = in ? a.bcs[col.z + z + 1] - b0 : 0;
+      }
+      bool full = false;
+      for (; __any_sync(kAll, v - gl < nb + np); v += kStep) {
+        if ((full = __any_sync(kAll, cnt > kNlistMax && rebuild))) break;
+#pragma unroll
+        for (int u = 0; u < kStep; u += G) {
+          const int w = v + u;
+          bool hit = false;
+          int e = 0;
+          if (w < nb) {
+            e = -(b0 + w) - 1;
+            const float4 pb = a.bpos[b0 + w];
+            const float bx = t.x.x - pb.x, by = t.x.y - pb.y, bz = t.x.z - pb.z;
+            hit = !(__fmaf_rn(bx, bx, __fmaf_rn(by, by, __fmul_rn(bz, bz))) > Bs2);
+            walls |= hit;
+          } else if (w < nb + np) {
+            e = j0 + w - nb;
+            const float4 xj = a.xs[e];
+            const float dx = t.x.x - xj.x, dy = t.x.y - xj.y, dz = t.x.z - xj.z;
+            const float rs = rcs + xj.w;
+            hit = !(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))) > rs * rs * 1.0001f) && e != i;
+          }
+          const unsigned hb = gballot(hit);
+          if (hit) s_list[grp][cnt + __popc(hb & glt)] = e;
+          cnt += __popc(hb);
+        }
+      }
+      if (full) break;
+      v = gl;
+      seg += cells ? 1 : 3;
+    }
+    const bool done = seg >= 27;
+    const unsigned wb = gballot(walls);  // (every lane votes; kept lists carry the flag in all of theirs)
+    walls = wb != 0;
+    // a list that overflowed runs as far as it goes; once the scan is done,
+    // every list runs (and, if it holds every candidate, is kept)
+    const bool filled = rebuild && cnt > kNlistMax;
+    over |= filled;
+    __syncwarp();
+    if (done && rebuild) {
+      if (!over)
+        for (int k = gl; k < cnt; k += G) row[k * a.li_step] = s_list[grp][k];
+      if (gl == 0) {
+        a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, over ? -1 : cnt | (walls ? kNlistWalls : 0));
+        a.nl_acc[i] = 0.0f;
+      }
+    }
+    const int n = done || filled ? cnt : 0;
+    if (walls && n > 0) target_walls(a, t);
+    for (int k0 = 0; __any_sync(kAll, k0 < n); k0 += G) {
+      Share s;
+      bool con = false, back = false;
+      if (k0 + gl < n) {
+        const int e = rebuild ? s_list[grp][k0 + gl] : row[k0 + gl];
+        if (e >= 0) {
+          con = pair_contact<MM>(a, t, e, a.xs[e], a.inv_m[e], s, back);
+        } else {
+          const float4 pb = a.bpos[-e - 1];
+          con = wall_near(t, pb) && wall_contact<MM>(a, t, pb, s);
+        }
+      }
+      const unsigned cb = gballot(con);
+      const int num = __popc(cb);
+      s_loc += __popc(gballot(back));
+      c += num;
+      if (con) {
+        float* sh = &s_share[grp][__popc(cb & glt)];
+        sh[0] = s.dp.x;
+        sh[G] = s.dp.y;
+        sh[2 * G] = s.dp.z;
+        if (MM & 2) {
+          sh[3 * G] = s.df.x;
+          sh[4 * G] = s.df.y;
+          sh[5 * G] = s.df.z;
+        }
+      }
+      __syncwarp();
+      if (gl < NC) {
+        const float* sh = &s_share[grp][gl * G];
+        for (int k = 0; k < num; ++k) sum += sh[k];
+      }
+      __syncwarp();
+    }
+    if (done) break;
+    if (filled) cnt = 0;
+  }
+  if (act) {
+    float* out = reinterpret_cast<float*>(a.delta + i);
+    if (gl < 3) out[gl] = sum;
+    if (gl == 3) out[3] = __int_as_float((c & 0xffff) | (s_loc << 16));
+    if (MM & 2) {
+      out = reinterpret_cast<float*>(a.fdelta + i);
+      if (gl >= 3 && gl < 6) out[gl - 3] = sum;
+      if (gl == 6) out[3] = __int_as_float(c);
+    }
+  }
+  const int built = __syncthreads_count(rebuild && gl == 0);
+  if (threadIdx.x == 0 && built && queue != a.nl_over)  // (those are counted by the threads that left them)
+    atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)built);
   }
 }
 
@@ -710,6 +923,31 @@ gg_status window_table(gg_system* S, cudaStream_t st) {
   k_window_table<<<blocks_for(n, 128), 128, 0, st>>>(n, S->grid.L, S->window);
   GG_CUDA(cudaGetLastError());
   return GG_OK;
+}
+
+// Systems up to this size give every particle a group of lanes.  Measured
+// against the thread kernels with their queues left to groups, per pass:
+// 51,000 particles (10 listed each) 1.66 against 1.82 ms, 125,000 in a dense
+// pile (28 listed) 2.78 against 3.07 ms, but 144,000 loosely packed (6
+// listed) 11.3 against 9.2 ms and 643,000 (23 listed) 8.7 against 5.6 ms:
+// the line lies where a thread to a particle starts to fill the chip.
+constexpr int64_t kGroupMax = 100000;
+
+// Queues up to this length are rebuilt by groups (30,000 to 240,000 measured
+// the same; 15,000 lost 30 % on 643,000 settled particles).
+constexpr int kGroupQueue = 65536;
+
+// Lanes to a particle: 1,000 particles ran a frame in 925 us with 32, 950
+// with 16 and 1,000 with 8; 32,768 particles in 1,136, 958 and 914 us.
+constexpr int64_t kGroup32Max = 4096, kGroup16Max = 16384;
+
+template <int G>
+static void launch_group(const SweepArgs& a, int mm, cudaStream_t st) {
+  auto kern = mm == 0   ? k_sweep_group<0, G, false>
+              : mm == 1 ? k_sweep_group<1, G, false>
+              : mm == 2 ? k_sweep_group<2, G, false>
+                        : k_sweep_group<3, G, false>;
+  kern<<<blocks_for(a.n, kGroupThreads / G), kGroupThreads, 0, st>>>(a);
 }
 
 gg_status sweep(gg_system* S, int it, cudaStream_t st) {
@@ -745,7 +983,9 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st) {
   a.nl_acc = S->g.nl_acc;
   a.nl_queue = S->g.nl_queue;
   a.cell_inc = S->g.cell_inc;
-  a.cap = (int)S->cap;
+  a.nl_over = S->g.split_slot;  // (scratch of the split, free during the sweeps)
+  a.li_row = a.li_step = 0;
+  a.group_queue = 0;
   a.skin = S->nl_skin;
   a.div_yz = make_udiv((uint32_t)(S->grid.ny * S->grid.nz));
   a.div_z = make_udiv((uint32_t)S->grid.nz);
@@ -762,7 +1002,16 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st) {
   if (S->tune.sweep_variant == 1) {
     auto kern = (mm == 0 ? k_sweep<0> : mm == 1 ? k_sweep<1> : mm == 2 ? k_sweep<2> : k_sweep<3>);
     kern<<<blocks_for(S->n, 256), 256, 0, st>>>(a);
+  } else if (S->g.nl_idx && S->n <= kGroupMax) {
+    a.li_row = kNlistMax;
+    a.li_step = 1;
+    if (S->n <= kGroup32Max) launch_group<32>(a, mm, st);
+    else if (S->n <= kGroup16Max) launch_group<16>(a, mm, st);
+    else launch_group<8>(a, mm, st);
   } else if (S->g.nl_idx) {
+    a.li_row = 1;
+    a.li_step = (size_t)S->cap;
+    a.group_queue = kGroupQueue;
     auto build = (mm == 0 ? k_sweep_nlist_build<0> : mm == 1 ? k_sweep_nlist_build<1> : mm == 2 ? k_sweep_nlist_build<2> : k_sweep_nlist_build<3>);
     if (it == 0) {
       build<<<blocks_for(S->n, kBuildThreads), kBuildThreads, 0, st>>>(a, 0);
@@ -774,6 +1023,10 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st) {
       build<<<nb, kBuildThreads, 0, st>>>(a, 1);
       count_launches(S, 1);
     }
+    // short queues, and what a list does not hold
+    auto rest = (mm == 0 ? k_sweep_group<0, 8, true> : mm == 1 ? k_sweep_group<1, 8, true> : mm == 2 ? k_sweep_group<2, 8, true> : k_sweep_group<3, 8, true>);
+    rest<<<S->num_sms * 3, kGroupThreads, 0, st>>>(a);
+    count_launches(S, 1);
   } else {
     auto kern = (mm == 0 ? k_sweep_list<0> : mm == 1 ? k_sweep_list<1> : mm == 2 ? k_sweep_list<2> : k_sweep_list<3>);
     kern<<<blocks_for(S->n, kWarpThreads), kWarpThreads, 0, st>>>(a);
