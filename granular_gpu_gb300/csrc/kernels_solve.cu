@@ -7,6 +7,7 @@
 // one apply kernel with no fill kernels; final_update (:193-270) and the
 // adaptive_last_step fill (:103-108) become one finalize kernel.
 #include "common.cuh"
+#include "f32x2.cuh"
 
 namespace gg {
 
@@ -326,8 +327,73 @@ struct UpArgs {
   const float4* __restrict__ bpos;
   const int32_t* __restrict__ cs;
   const int32_t* __restrict__ bcs;
+  const float4* __restrict__ pair_a;  // two particles to an entry (k_pair_particles)
+  const float4* __restrict__ pair_b;
+  const float4* __restrict__ pair_c;
+  float one;                          // 1, not known to the compiler (add_product2)
   float r9, cut2, gdt_y, dtu, brad, brad_cut2, repulsion, vmax, floor_y, floor_fric, bdamp, band, gdamp;
 };
+
+// The wall particles of a stencil column: the repulsion near them.
+__device__ __forceinline__ void up_walls(const UpArgs& a, float3 p, int k0, int nc, bool& near_b, float3& rep) {
+  const int k1 = a.bcs[k0 + nc];
+  for (int k = a.bcs[k0]; k < k1; ++k) {
+    const float4 b = a.bpos[k];
+    const float3 tb = make_float3(p.x - b.x, p.y - b.y, p.z - b.z);
+    const float dd = dot3(tb, tb);
+    if (dd > a.brad_cut2) continue;
+    const float dis = sqrtf(dd);
+    if (dis < a.brad) {
+      near_b = true;
+      const float3 nrm = div3s(tb, dis + 1e-6f);
+      const float force = a.repulsion * (a.brad - dis) / a.brad;
+      rep = add3(rep, mul3s(nrm, force));
+    }
+  }
+}
+
+// The render point's new velocity and position from its sums.
+__device__ __forceinline__ void up_finish(const UpArgs& a, int i, float4 p4, float3 wv, float3 rep, float gw,
+                                          float maxw, bool near_b) {
+  const float3 p = f3(p4);
+  const float4 uv4 = a.uvel[i];
+  const float3 uv = f3(uv4);
+  const float3 gdt = make_float3(0.0f * a.dtu, a.gdt_y, 0.0f * a.dtu);
+  float3 nv;
+  if (gw > 1e-6f) {
+    wv = div3s(wv, gw);
+    const float alpha = fmaxf(0.0f, 1.0f - maxw);
+    nv = add3(smul3(alpha, add3(uv, gdt)), smul3(1.0f - alpha, wv));
+  } else {
+    nv = add3(uv, gdt);
+    if (near_b) {
+      nv = mul3s(nv, a.bdamp);
+      if (p.y < a.band) nv.y = nv.y * a.gdamp;
+    }
+  }
+  nv = add3(nv, rep);
+  nv.x = fmaxf(-a.vmax, fminf(nv.x, a.vmax));
+  nv.y = fmaxf(-a.vmax, fminf(nv.y, a.vmax));
+  nv.z = fmaxf(-a.vmax, fminf(nv.z, a.vmax));
+  if (isnan(nv.x) || isnan(nv.y) || isnan(nv.z)) nv = make_float3(0.f, 0.f, 0.f);
+  float3 up = add3(p, mul3s(nv, a.dtu));
+  if (up.y < a.floor_y) {
+    up.y = a.floor_y;
+    nv.y = 0.0f;
+    nv.x = nv.x * a.floor_fric;
+    nv.z = nv.z * a.floor_fric;
+  }
+  if (up.x < 0.0f) {
+    up.x = 0.0f;
+    nv.x = 0.0f;
+  }
+  if (up.z < 0.0f) {
+    up.z = 0.0f;
+    nv.z = 0.0f;
+  }
+  a.uvel[i] = make_float4(nv.x, nv.y, nv.z, 0.f);
+  a.upos[i] = make_float4(up.x, up.y, up.z, p4.w);
+}
 
 // update_upsampled_cuda, Solver.cu:1244-1369.  Candidates beyond the kernel
 // support (w = 0 exactly) are skipped; adding +0 would not change a sum.
@@ -397,60 +463,90 @@ __global__ void __launch_bounds__(256, 6) k_upsample(UpArgs a) {
         }
       }
     }
-    const int k1 = a.bcs[k0 + nc];
-    for (int k = a.bcs[k0]; k < k1; ++k) {
-      const float4 b = a.bpos[k];
-      const float3 tb = make_float3(p.x - b.x, p.y - b.y, p.z - b.z);
-      const float dd = dot3(tb, tb);
-      if (dd > a.brad_cut2) continue;
-      const float dis = sqrtf(dd);
-      if (dis < a.brad) {
-        near_b = true;
-        const float3 nrm = div3s(tb, dis + 1e-6f);
-        const float force = a.repulsion * (a.brad - dis) / a.brad;
-        rep = add3(rep, mul3s(nrm, force));
-      }
-    }
+    up_walls(a, p, k0, nc, near_b, rep);
   });
-  const float4 uv4 = a.uvel[i];
-  const float3 uv = f3(uv4);
-  const float3 gdt = make_float3(0.0f * a.dtu, a.gdt_y, 0.0f * a.dtu);
-  float3 nv;
-  if (gw > 1e-6f) {
-    wv = div3s(wv, gw);
-    const float alpha = fmaxf(0.0f, 1.0f - maxw);
-    nv = add3(smul3(alpha, add3(uv, gdt)), smul3(1.0f - alpha, wv));
-  } else {
-    nv = add3(uv, gdt);
-    if (near_b) {
-      nv = mul3s(nv, a.bdamp);
-      if (p.y < a.band) nv.y = nv.y * a.gdamp;
-    }
-  }
-  nv = add3(nv, rep);
-  nv.x = fmaxf(-a.vmax, fminf(nv.x, a.vmax));
-  nv.y = fmaxf(-a.vmax, fminf(nv.y, a.vmax));
-  nv.z = fmaxf(-a.vmax, fminf(nv.z, a.vmax));
-  if (isnan(nv.x) || isnan(nv.y) || isnan(nv.z)) nv = make_float3(0.f, 0.f, 0.f);
-  float3 up = add3(p, mul3s(nv, a.dtu));
-  if (up.y < a.floor_y) {
-    up.y = a.floor_y;
-    nv.y = 0.0f;
-    nv.x = nv.x * a.floor_fric;
-    nv.z = nv.z * a.floor_fric;
-  }
-  if (up.x < 0.0f) {
-    up.x = 0.0f;
-    nv.x = 0.0f;
-  }
-  if (up.z < 0.0f) {
-    up.z = 0.0f;
-    nv.z = 0.0f;
-  }
-  a.uvel[i] = make_float4(nv.x, nv.y, nv.z, 0.f);
-  a.upos[i] = make_float4(up.x, up.y, up.z, p4.w);
+  up_finish(a, i, p4, wv, rep, gw, maxw, near_b);
 }
 
+// The same for a support that reaches every candidate of the stencil, on
+// packed pairs of candidates: k_upsample<true> is bound by the issue of
+// about 48 instructions a candidate, this form issues 32 and is bound by the
+// FP32 pipe (65 % active) and the loads.  10.56 to 9.33 ms per launch on the
+// 8.4 M column (33.5 M render points, 263 candidates each; 0.06 ms of
+// pairing included).  The particles come two to an entry, so three loads
+// bring two of them in the pairs that the packed operations take; the sums
+// stay single and in candidate order, so the results are the same bits.  A
+// column's first and last entry may hold a particle that is not of the
+// column: it takes no part in the sums.
+__global__ void __launch_bounds__(256, 4) k_upsample_pairs(UpArgs a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  const Grid g = a.g;
+  const float4 p4 = a.upos[i];
+  const float3 p = f3(p4);
+  float3 wv = make_float3(0.f, 0.f, 0.f), rep = make_float3(0.f, 0.f, 0.f);
+  float gw = 0.f, maxw = 0.f;
+  bool near_b = false;
+  const f32x2 px = pack2(p.x, p.x), py = pack2(p.y, p.y), pz = pack2(p.z, p.z);
+  const f32x2 neg_r9 = pack2(-a.r9, -a.r9), one = pack2(1.0f, 1.0f), ones = pack2(a.one, a.one);
+  for_each_stencil_column(g, floor_cell(g, p), [&](int k0, int nc) {
+    const int j0 = a.cs[k0], j1 = a.cs[k0 + nc];
+    const int e1 = (j1 + 1) >> 1;
+#pragma unroll 2
+    for (int e = j0 >> 1; e < e1; ++e) {
+      const float4 A = a.pair_a[e], B = a.pair_b[e], C = a.pair_c[e];
+      // the reference's weight (Solver.cu:1281-1287); p - x as p + (-x) and
+      // 1 - d^2 r9 as 1 + d^2 (-r9), which round alike
+      const f32x2 dx = add2(px, pack2(A.x, A.y)), dy = add2(py, pack2(A.z, A.w)), dz = add2(pz, pack2(B.x, B.y));
+      const f32x2 dd = add_product2(mul2(dz, dz), ones, add_product2(mul2(dx, dx), ones, mul2(dy, dy)));
+      float d0, d1;
+      unpack2(dd, d0, d1);
+      // (below 1e-30 the weight is 1 to the last bit either way)
+      const f32x2 dis = sqrt2(pack2(max_nan(d0, 1e-30f), max_nan(d1, 1e-30f)));
+      const f32x2 t1 = add_product2(mul2(mul2(dis, dis), neg_r9), ones, one);
+      const f32x2 w2 = mul2(mul2(t1, t1), t1);
+      float w0, w1;
+      unpack2(w2, w0, w1);
+      w0 = fmaxf(0.0f, w0);
+      w1 = fmaxf(0.0f, w1);
+      const f32x2 w = pack2(w0, w1);
+      float x0, x1, y0, y1, z0, z1;
+      unpack2(mul2(w, pack2(B.z, B.w)), x0, x1);
+      unpack2(mul2(w, pack2(C.x, C.y)), y0, y1);
+      unpack2(mul2(w, pack2(C.z, C.w)), z0, z1);
+      if (2 * e >= j0) {
+        gw += w0;
+        wv.x += x0;
+        wv.y += y0;
+        wv.z += z0;
+        maxw = fmaxf(maxw, w0);
+      }
+      if (2 * e + 1 < j1) {
+        gw += w1;
+        wv.x += x1;
+        wv.y += y1;
+        wv.z += z1;
+        maxw = fmaxf(maxw, w1);
+      }
+    }
+    up_walls(a, p, k0, nc, near_b, rep);
+  });
+  up_finish(a, i, p4, wv, rep, gw, maxw, near_b);
+}
+
+// Two particles to an entry: their negated positions and their velocities,
+// a coordinate's two values side by side.
+__global__ void __launch_bounds__(256) k_pair_particles(int n, const float4* __restrict__ pos,
+                                                        const float4* __restrict__ vel, float4* __restrict__ pa,
+                                                        float4* __restrict__ pb, float4* __restrict__ pc) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (2 * e >= n) return;
+  const int j = min(2 * e + 1, n - 1);  // (an odd last particle fills both halves)
+  const float4 x0 = pos[2 * e], x1 = pos[j], v0 = vel[2 * e], v1 = vel[j];
+  pa[e] = make_float4(-x0.x, -x1.x, -x0.y, -x1.y);
+  pb[e] = make_float4(-x0.z, -x1.z, v0.x, v1.x);
+  pc[e] = make_float4(v0.y, v1.y, v0.z, v1.z);
+}
 
 gg_status upsample(gg_system* S, cudaStream_t st) {
   if (S->nu <= 0) return GG_OK;
@@ -482,7 +578,24 @@ gg_status upsample(gg_system* S, cudaStream_t st) {
   const float reach2 = 12.0f * S->grid.L * S->grid.L * 1.001f;
   const bool all_in = reach2 * S->P.up_inv_h2 < 0.999f;
   prof_begin(S, PC_UPSAMPLE, st);
-  if (all_in) k_upsample<true><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
+  // the packed form wants memory for the pairs and a support that is one
+  // (with a negative 1/h^2, infinite distances would weigh)
+  if (all_in && S->P.up_inv_h2 > 0.0f && S->g.nl_idx) {
+    // the contact lists of the substep are done with: their memory holds the
+    // pairs (24 of its 256 bytes a particle)
+    const int64_t np = (S->n + 1) / 2;
+    float4* pairs = reinterpret_cast<float4*>(S->g.nl_idx);
+    a.pair_a = pairs;
+    a.pair_b = pairs + np;
+    a.pair_c = pairs + 2 * np;
+    a.one = 1.0f;
+    if (np > 0) {
+      k_pair_particles<<<blocks_for(np, 256), 256, 0, st>>>((int)S->n, a.gpos, a.gvel, pairs, pairs + np,
+                                                            pairs + 2 * np);
+      count_launches(S, 1);
+    }
+    k_upsample_pairs<<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
+  } else if (all_in) k_upsample<true><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
   else k_upsample<false><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
   count_launches(S, 1);
   prof_end(S, PC_UPSAMPLE, S->nu, st);
