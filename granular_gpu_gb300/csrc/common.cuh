@@ -186,6 +186,11 @@ __device__ __forceinline__ void block_max_bits_any(unsigned int* dst, unsigned i
   __syncthreads();  // s_max is reused by the next call
 }
 
+// The residual of a solve: the mean penetration over the contacts.
+__host__ __device__ __forceinline__ float residual_mean(double sum, unsigned int count) {
+  return count ? (float)(sum / (double)count) : 0.0f;
+}
+
 __device__ __forceinline__ unsigned int lanemask_lt() {
   unsigned int m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

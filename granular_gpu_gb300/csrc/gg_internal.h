@@ -42,6 +42,13 @@ inline UDiv make_udiv(uint32_t d) {
 // Scalars that live on the device so a substep needs no host round trip.
 constexpr int kMaxSweeps = 2048;  // sweeps per substep (stabilisation + Jacobi)
 
+// Residual mode: the penetrations at x* that a sweep saw.
+struct ResidualSlot {
+  double sum;                // of the positive ones
+  unsigned int count;        // their number (particle pairs counted once per side, walls)
+  unsigned int most_bits;    // the largest (float bits)
+};
+
 struct DevScalars {
   unsigned int rmax_bits;      // max contact radius (float bits), this step
   unsigned int inc_bits[kMaxSweeps];  // per sweep: max |x* increment| per axis (float bits)
@@ -50,6 +57,8 @@ struct DevScalars {
   unsigned int tile_fallback;  // sweep blocks that could not use the shared-memory tile
   int nl_queued[kMaxSweeps];          // per sweep: particles whose contact list is rebuilt
   int nl_over[kMaxSweeps];     // per sweep: particles with more candidates than a list holds
+  ResidualSlot res[kMaxSweeps];  // residual mode, per sweep
+  int res_done;                // residual mode: 1 + the sweep whose x* met the target (later sweeps do nothing)
   unsigned int pen_bits;       // residual mode: largest penetration (float bits)
   unsigned int pen_count;      // residual mode: contacts (particle pairs counted once per side, walls)
   double pen_sum;              // residual mode: sum of their penetrations
@@ -296,11 +305,17 @@ gg_status reorder_upsampled(gg_system* S, const uint32_t* perm, cudaStream_t st)
 gg_status radii_all(gg_system* S, cudaStream_t st);
 gg_status predict(gg_system* S, cudaStream_t st);
 gg_status window_table(gg_system* S, cudaStream_t st);
-gg_status sweep(gg_system* S, int it, cudaStream_t st);
+// res (only where sweep_sums_residual holds): the sweep also sums the
+// penetrations at x* there, and does nothing once scal->res_done is set.
+gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res = nullptr);
+bool sweep_sums_residual(const gg_system* S);
 // last: write the constraint counts (the substep's last sweep, or every
 // sweep of the residual mode); more: another sweep may follow, so record the
 // per-cell increments its contact lists are checked against.
-gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStream_t st);
+// res: apply nothing (and set scal->res_done) if the sweep's penetrations
+// are within gg_params.target_residual.
+gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStream_t st,
+                const ResidualSlot* res = nullptr);
 gg_status finalize(gg_system* S, cudaStream_t st);
 gg_status upsample(gg_system* S, cudaStream_t st);
 gg_status explosion(gg_system* S, float force, cudaStream_t st);
@@ -316,6 +331,7 @@ gg_status warm_start_apply(gg_system* S, cudaStream_t st);
 gg_status warm_start_record(gg_system* S, cudaStream_t st);
 gg_status warm_start_target(gg_system* S, cudaStream_t st);
 gg_status residual(gg_system* S, cudaStream_t st, float* out);
+gg_status solve_to_residual(gg_system* S, int first, int cap, cudaStream_t st, int* sweeps, float* out);
 
 // stats
 gg_status stats_compute(gg_system* S, gg_stats_t* out);

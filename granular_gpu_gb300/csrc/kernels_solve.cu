@@ -91,6 +91,14 @@ struct PlaneArgs {
   const float2* __restrict__ scene_mu;
 };
 
+// Residual mode: the sweep's penetrations and the target they are held to.
+struct ResidualArgs {
+  const ResidualSlot* __restrict__ res;  // null: apply always
+  volatile int* done;
+  float target;
+  int it;
+};
+
 // change_position_functor (Solver.cu:403-414): x* += delta / max(1, n); in
 // the stabilisation sweeps x as well (:457-460).
 //
@@ -112,8 +120,18 @@ __global__ void __launch_bounds__(256) k_apply(int n, float4* __restrict__ xs, f
                         unsigned int* __restrict__ inc_bits, unsigned int* __restrict__ inc_norm_bits,
                         const uint32_t* __restrict__ keys,
                         uint32_t* __restrict__ cell_inc, int C, int nz, UDiv div_z, PlaneArgs pa,
-                        const float4* __restrict__ fdelta, float* __restrict__ pn) {
+                        const float4* __restrict__ fdelta, float* __restrict__ pn, ResidualArgs ra) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ra.res) {
+    // residual mode: x* is left as it is once the sweep found it within the
+    // target (the counts that it handed to others are taken back)
+    if (*ra.done && *ra.done <= ra.it) return;
+    if (!(residual_mean(ra.res->sum, ra.res->count) > ra.target)) {
+      if (i < n) s_extra[i] = 0;
+      if (i == 0) *ra.done = ra.it + 1;
+      return;
+    }
+  }
   unsigned int bits = 0, nbits = 0;
   uint32_t key = 0xffffffffu;
   if (i < n) {
@@ -231,7 +249,7 @@ __global__ void __launch_bounds__(256) k_apply(int n, float4* __restrict__ xs, f
   block_max_bits_any(inc_norm_bits, nbits);
 }
 
-gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStream_t st) {
+gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStream_t st, const ResidualSlot* res) {
   if (S->n <= 0) return GG_OK;
   prof_begin(S, PC_APPLY, st);
   // a listed sweep after this one (more) reads the per-cell increments
@@ -254,7 +272,8 @@ gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStrea
                                                  last ? 1 : 0, &S->scal->inc_bits[it], &S->scal->inc_norm_bits[it],
                                                  S->g.keys, cell_inc,
                                                  S->grid.C, S->grid.nz, make_udiv((uint32_t)S->grid.nz), pa,
-                                                 pa.coulomb ? S->g.fdelta : nullptr, S->g.pn);
+                                                 pa.coulomb ? S->g.fdelta : nullptr, S->g.pn,
+                                                 ResidualArgs{res, &S->scal->res_done, S->P.target_residual, it});
   count_launches(S, 1);
   prof_end(S, PC_APPLY, S->n, st);
   GG_CUDA(cudaGetLastError());

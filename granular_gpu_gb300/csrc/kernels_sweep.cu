@@ -26,6 +26,7 @@
 // particle scan the autotuner may pick where lists do not pay.
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -58,6 +59,7 @@ struct SweepArgs {
   int32_t* __restrict__ nl_over;   // particles with more candidates than a list holds, left to the groups
   size_t li_row, li_step;          // entry k of particle i's list: nl_idx[i * li_row + k * li_step]
   const uint32_t* __restrict__ cell_inc;
+  ResidualSlot* res;               // residual mode: this sweep's penetrations (kernels with bit 2 of MM)
   int group_queue;                 // queues up to this length are rebuilt by groups
   float skin;
   float eabs;    // bound on the rounding of one position update
@@ -76,7 +78,8 @@ struct SweepArgs {
 
 // The kernels' template argument MM: bit 0 the math mode (0 CUDA's
 // functions, 1 rounded once from double), bit 1 the contact law (0 the
-// reference's, 1 Coulomb friction).
+// reference's, 1 Coulomb friction), bit 2 the residual mode (also sum the
+// penetrations at x*, which the candidates of the sweep hold all of).
 
 // Which of the three cell columns [c-1, c, c+1] along one axis can hold a
 // partner: bit k set for offset k-1.  Cells are [cL, (c+1)L) in binning
@@ -285,6 +288,58 @@ __device__ __forceinline__ bool pair_contact(const SweepArgs& a, const Target& t
   return true;
 }
 
+// Residual mode: a thread's penetrations r_i + r_j - |x_i - x_j| over the
+// pairs in the sweep's stencil and (0.01 + max(r_i, 0.01)) - |x - b| over
+// wall particles, as k_residual takes them (a pair counts once from each
+// side; the mean is unchanged by that).  Every positive one is a listed
+// candidate, since lists reach past contact.
+struct Penetration {
+  float sum = 0.0f, most = 0.0f;
+  unsigned int count = 0;
+};
+__device__ __forceinline__ void add_penetration(const Target& t, int e, float4 p, Penetration& u) {
+  const float dx = t.x.x - p.x, dy = t.x.y - p.y, dz = t.x.z - p.z;
+  const float R = e >= 0 ? t.rc + p.w : t.Bf;
+  const float d2 = dx * dx + dy * dy + dz * dz;
+  if (d2 < R * R) {
+    const float pen = R - sqrtf(d2);
+    u.most = fmaxf(u.most, pen);
+    u.sum += pen;
+    ++u.count;
+  }
+}
+// A block's penetrations into its sweep's slot (every thread calls it).
+__device__ __forceinline__ void store_penetration(const SweepArgs& a, const Penetration& u) {
+  __shared__ float s_sum[8];
+  __shared__ unsigned int s_count[8], s_most[8];
+  float ws = u.sum;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+  const unsigned int wc = __reduce_add_sync(0xffffffffu, u.count);
+  const unsigned int wm = __reduce_max_sync(0xffffffffu, __float_as_uint(u.most));
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    s_sum[w] = ws;
+    s_count[w] = wc;
+    s_most[w] = wm;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double bs = 0.0;
+    unsigned int bc = 0, bm = 0;
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+      bs += (double)s_sum[k];
+      bc += s_count[k];
+      bm = max(bm, s_most[k]);
+    }
+    if (bc) {
+      atomicAdd(&a.res->sum, bs);
+      atomicAdd(&a.res->count, bc);
+      atomicMax(&a.res->most_bits, bm);
+    }
+  }
+}
+
 // The running sums of one thread's target.
 struct Sums {
   float3 dp = {0.f, 0.f, 0.f}, df = {0.f, 0.f, 0.f};
@@ -466,7 +521,7 @@ __device__ __forceinline__ void fetch_entry(const SweepArgs& a, int e, float4& p
 
 template <int MM, class EntryF>
 __device__ __forceinline__ void apply_entries(const SweepArgs& a, const Target& t, int cnt, EntryF&& entry,
-                                              Sums& u) {
+                                              Sums& u, Penetration& pen) {
   if (cnt <= 0) return;
   int e_next = entry(0);
   int e_after = cnt > 1 ? entry(1) : INT_MIN;
@@ -480,6 +535,7 @@ __device__ __forceinline__ void apply_entries(const SweepArgs& a, const Target& 
     e_next = e_after;
     fetch_entry(a, e_next, p_next, im_next);
     e_after = (k + 2 < cnt) ? entry(k + 2) : INT_MIN;
+    if (MM & 4) add_penetration(t, e, p, pen);
     if (e >= 0) add_pair<MM>(a, t, e, p, im, u);
     else if (wall_near(t, p)) add_wall<MM>(a, t, p, u);
   }
@@ -535,8 +591,10 @@ __device__ __forceinline__ float nlist_cell_bound(const SweepArgs& a, int3 q, ui
 template <int MM>
 __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(SweepArgs a) {
   const Grid& g = a.g;
+  if ((MM & 4) && a.scal->res_done) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool rebuild = false;
+  Penetration pen;
   if (i < a.n) {
     const float4 xi4 = a.xs[i];
     const int3 q = trunc_cell(g, f3(xi4));
@@ -557,7 +615,7 @@ __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(SweepArgs a) {
       if (m.w & kNlistWalls) target_walls(a, t);
       Sums u;
       const int32_t* __restrict__ li = a.nl_idx + i;
-      apply_entries<MM>(a, t, m.w & kNlistCount, [&](int k) { return __ldcs(li + k * a.li_step); }, u);
+      apply_entries<MM>(a, t, m.w & kNlistCount, [&](int k) { return __ldcs(li + k * a.li_step); }, u, pen);
       store_sums<MM>(a, i, u);
     } else {
       rebuild = true;
@@ -582,6 +640,7 @@ __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(SweepArgs a) {
   }
   __syncthreads();
   if (rebuild) a.nl_queue[s_base + s_cnt[w] + __popc(bal & lanemask_lt())] = i;
+  if (MM & 4) store_penetration(a, pen);
 }
 
 // List build: scan the 27 cells in the reference order, write the
@@ -598,6 +657,8 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArg
   const int lane = threadIdx.x & 31;
   const int total = queued ? a.scal->nl_queued[a.it] : a.n;
   if (queued && total <= a.group_queue) return;  // the groups take a short queue
+  if ((MM & 4) && a.scal->res_done) return;
+  Penetration pen;
   for (int base = blockIdx.x * kBuildThreads; base < total; base += gridDim.x * kBuildThreads) {
     const int slot = base + threadIdx.x;
     const bool act = slot < total;
@@ -678,9 +739,10 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArg
     if (walls) target_walls(a, t);
     Sums u;
     // the list this thread just wrote (its own stores: read back in order)
-    apply_entries<MM>(a, t, cnt, [&](int k) { return li[k * a.li_step]; }, u);
+    apply_entries<MM>(a, t, cnt, [&](int k) { return li[k * a.li_step]; }, u, pen);
     store_sums<MM>(a, i, u);
   }
+  if (MM & 4) store_penetration(a, pen);
 }
 
 // ------------------------------------------------------------ group sweep
@@ -721,6 +783,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
     const unsigned b = __ballot_sync(kAll, p);
     return G == 32 ? b : (b >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u);
   };
+  if ((MM & 4) && a.scal->res_done) return;
+  Penetration pen;
   int total = a.n;
   const int32_t* queue = nullptr;
   if (kQueue) {
@@ -848,12 +912,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
       bool con = false, back = false;
       if (k0 + gl < n) {
         const int e = rebuild ? s_list[grp][k0 + gl] : row[k0 + gl];
-        if (e >= 0) {
-          con = pair_contact<MM>(a, t, e, a.xs[e], a.inv_m[e], s, back);
-        } else {
-          const float4 pb = a.bpos[-e - 1];
-          con = wall_near(t, pb) && wall_contact<MM>(a, t, pb, s);
-        }
+        const float4 p = e >= 0 ? a.xs[e] : a.bpos[-e - 1];
+        if (MM & 4) add_penetration(t, e, p, pen);
+        if (e >= 0) con = pair_contact<MM>(a, t, e, p, a.inv_m[e], s, back);
+        else con = wall_near(t, p) && wall_contact<MM>(a, t, p, s);
       }
       const unsigned cb = gballot(con);
       const int num = __popc(cb);
@@ -894,6 +956,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
   if (threadIdx.x == 0 && built && queue != a.nl_over)  // (those are counted by the threads that left them)
     atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)built);
   }
+  if (MM & 4) store_penetration(a, pen);
 }
 
 // The window of a cell coordinate c: [lo, hi) holds exactly the positions x
@@ -941,16 +1004,33 @@ constexpr int kGroupQueue = 65536;
 // with 16 and 1,000 with 8; 32,768 particles in 1,136, 958 and 914 us.
 constexpr int64_t kGroup32Max = 4096, kGroup16Max = 16384;
 
+// A sweep kernel by its template argument (math mode 1 sums no penetrations:
+// sweep_sums_residual).
+#define GG_SWEEP_KERNEL(MMVAL, ...)                                                                       \
+  [&]() {                                                                                                 \
+    auto pick = [](auto m) { constexpr int MM = decltype(m)::value; return &__VA_ARGS__; };               \
+    using std::integral_constant;                                                                         \
+    switch (MMVAL) {                                                                                      \
+      case 0: return pick(integral_constant<int, 0>());                                                   \
+      case 1: return pick(integral_constant<int, 1>());                                                   \
+      case 2: return pick(integral_constant<int, 2>());                                                   \
+      case 3: return pick(integral_constant<int, 3>());                                                   \
+      case 4: return pick(integral_constant<int, 4>());                                                   \
+      default: return pick(integral_constant<int, 6>());                                                  \
+    }                                                                                                     \
+  }()
+
 template <int G>
 static void launch_group(const SweepArgs& a, int mm, cudaStream_t st) {
-  auto kern = mm == 0   ? k_sweep_group<0, G, false>
-              : mm == 1 ? k_sweep_group<1, G, false>
-              : mm == 2 ? k_sweep_group<2, G, false>
-                        : k_sweep_group<3, G, false>;
+  auto kern = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, G, false>);
   kern<<<blocks_for(a.n, kGroupThreads / G), kGroupThreads, 0, st>>>(a);
 }
 
-gg_status sweep(gg_system* S, int it, cudaStream_t st) {
+bool sweep_sums_residual(const gg_system* S) {
+  return S->g.nl_idx && S->tune.sweep_variant == 0 && !S->P.math_mode && S->n > 0;
+}
+
+gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
   if (S->n <= 0) return GG_OK;
   SweepArgs a;
   a.g = S->grid;
@@ -977,7 +1057,8 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st) {
   const bool coulomb = S->P.contact_law == 1;
   a.pos0 = coulomb ? S->g.pos[S->g.cur] : nullptr;
   a.fdelta = coulomb ? S->g.fdelta : nullptr;
-  const int mm = (S->P.math_mode ? 1 : 0) | (coulomb ? 2 : 0);  // the kernels' template argument
+  const int mm = (S->P.math_mode ? 1 : 0) | (coulomb ? 2 : 0) | (res ? 4 : 0);  // the kernels' template argument
+  a.res = res;
   a.nl_idx = S->g.nl_idx;
   a.nl_meta = S->g.nl_meta;
   a.nl_acc = S->g.nl_acc;
@@ -1012,11 +1093,11 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st) {
     a.li_row = 1;
     a.li_step = (size_t)S->cap;
     a.group_queue = kGroupQueue;
-    auto build = (mm == 0 ? k_sweep_nlist_build<0> : mm == 1 ? k_sweep_nlist_build<1> : mm == 2 ? k_sweep_nlist_build<2> : k_sweep_nlist_build<3>);
+    auto build = GG_SWEEP_KERNEL(mm, k_sweep_nlist_build<MM>);
     if (it == 0) {
       build<<<blocks_for(S->n, kBuildThreads), kBuildThreads, 0, st>>>(a, 0);
     } else {
-      auto keep = (mm == 0 ? k_sweep_nlist_keep<0> : mm == 1 ? k_sweep_nlist_keep<1> : mm == 2 ? k_sweep_nlist_keep<2> : k_sweep_nlist_keep<3>);
+      auto keep = GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM>);
       const int tk = S->tune.keep_threads;
       keep<<<blocks_for(S->n, tk), tk, 0, st>>>(a);
       const int nb = std::min(blocks_for(S->n, kBuildThreads), S->num_sms * S->tune.build_blocks_per_sm);
@@ -1024,7 +1105,7 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st) {
       count_launches(S, 1);
     }
     // short queues, and what a list does not hold
-    auto rest = (mm == 0 ? k_sweep_group<0, 8, true> : mm == 1 ? k_sweep_group<1, 8, true> : mm == 2 ? k_sweep_group<2, 8, true> : k_sweep_group<3, 8, true>);
+    auto rest = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, 8, true>);
     rest<<<S->num_sms * 3, kGroupThreads, 0, st>>>(a);
     count_launches(S, 1);
   } else {

@@ -137,7 +137,9 @@ gg_status step_once(gg_system* S) {
     const int cap = std::max(0, std::min(S->P.max_sweeps, kMaxSweeps - stab));
     int k = 0;
     float res = 0.0f;
-    for (;;) {
+    if (sweep_sums_residual(S)) {
+      if ((rc = solve_to_residual(S, stab, cap, st, &k, &res)) != GG_OK) return rc;
+    } else for (;;) {
       if ((rc = residual(S, st, &res)) != GG_OK) return rc;
       if (!(res > S->P.target_residual) || k >= cap) break;
       if ((rc = sweep(S, stab + k, st)) != GG_OK) return rc;
@@ -169,7 +171,10 @@ gg_status step_once(gg_system* S) {
     S->merge_iter++;
     if ((rc = merge_count(S, st)) != GG_OK) return rc;
     if ((rc = split_and_compact(S, st)) != GG_OK) return rc;
-    GG_CUDA(cudaMemcpyAsync(S->scal_host, S->scal, sizeof(DevScalars), cudaMemcpyDeviceToHost, st));
+    // the counts at the end of the scalars (not the per-sweep tables)
+    constexpr size_t at = offsetof(DevScalars, error_word);
+    GG_CUDA(cudaMemcpyAsync(reinterpret_cast<char*>(S->scal_host) + at, reinterpret_cast<char*>(S->scal) + at,
+                            sizeof(DevScalars) - at, cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));
     const int64_t before = S->n;
     // k_compact wrote the other buffers unless nothing was removed or split
