@@ -20,19 +20,37 @@ namespace cg = cooperative_groups;
 
 // Prefilter of the neighbour test |d| <= 2 (r_i + r_j) with the surface-law
 // radius r_j: no contact radius (pos.w, which divides by the density
-// truncated to an integer) is below the surface-law radius, so with the
-// substep's largest contact radius w_max, a candidate beyond
-// R = 2.0002 (r_i + w_max), with a margin far above the roundings of a fused
-// dot product, fails the exact test.  Marks, in bit b, the candidates
-// c0 + b (b < cn <= 32) within R (R2 = R * R), leaving out i itself.
+// truncated to an integer) is below the surface-law radius, so a candidate
+// beyond R = 2.0002 (r_i + w), with a margin far above the roundings of a
+// fused dot product, fails the exact test, for its own contact radius w as
+// for the substep's largest.  The largest costs one comparison a candidate
+// and serves particles of about that size; among mixed masses the
+// candidate's own leaves a third as many to the exact test.  `keep` is a
+// squared distance within which all candidates pass (the density's), or
+// negative.
+__device__ __forceinline__ bool surface_near(float3 xi, float ri, float4 xj, float keep) {
+  const float3 d = sub3(xi, f3(xj));
+  const float dd = __fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, __fmul_rn(d.z, d.z)));
+  const float s = ri + xj.w;
+  return !(dd > s * s * 4.0008f && dd > keep);  // (a NaN passes)
+}
+
+// Marks, in bit b, the candidates c0 + b (b < cn <= 32) within reach,
+// leaving out i itself: of R2 = R^2 for the largest radius, or (mixed) of
+// their own.
 __device__ __forceinline__ unsigned surface_chunk_mask(const float4* __restrict__ pos, int c0, int cn, int i,
-                                                       float3 xi, float R2) {
+                                                       float3 xi, float ri, float R2, bool mixed, float keep) {
   unsigned mask = 0u;
+  if (mixed) {
 #pragma unroll 4
-  for (int b = 0; b < cn; ++b) {
-    const float3 d = sub3(xi, f3(pos[c0 + b]));
-    const float dd = __fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, __fmul_rn(d.z, d.z)));
-    mask |= (dd > R2 ? 0u : 1u) << b;
+    for (int b = 0; b < cn; ++b) mask |= (surface_near(xi, ri, pos[c0 + b], keep) ? 1u : 0u) << b;
+  } else {
+#pragma unroll 4
+    for (int b = 0; b < cn; ++b) {
+      const float3 d = sub3(xi, f3(pos[c0 + b]));
+      const float dd = __fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, __fmul_rn(d.z, d.z)));
+      mask |= (dd > R2 ? 0u : 1u) << b;
+    }
   }
   const unsigned self = (unsigned)(i - c0);
   if (self < 32u) mask &= ~(1u << self);
@@ -43,20 +61,86 @@ __device__ __forceinline__ unsigned surface_chunk_mask(const float4* __restrict_
 // vector's x and y), most aligned with it first.
 __constant__ int kTowards[9][2] = {{1, 1}, {1, 0}, {0, 1}, {0, 0}, {1, -1}, {-1, 1}, {0, -1}, {-1, 0}, {-1, -1}};
 
+struct SurfArgs {
+  Grid g;
+  int n;
+  const float4* __restrict__ pos;
+  const float* __restrict__ rs;
+  const int32_t* __restrict__ cs;
+  int32_t* __restrict__ surface;
+  float cone, cos_cone;
+  int min_nb;
+  const unsigned int* __restrict__ rmax_bits;
+  const float* __restrict__ mass;
+  float merge_cut;
+  float* __restrict__ ld_sum;
+  int32_t* __restrict__ ld_cnt;
+};
+
+// Warps with a particle this much smaller than the largest test candidates
+// against their own radius (1.05 to 1.5 measured the same).
+constexpr float kSurfMixed = 1.2f;
+
+// Whether neighbour j of a particle at xi lies within the cone around c.
+// acos(d) <= cone is decided from d alone away from cos(cone) (the margin of
+// 1e-5 on d is some 40 times the bound on acosf's error there and over the
+// rounding of cos_cone, computed on the host); near it acos is evaluated.
 template <int MM>
-__global__ void __launch_bounds__(256, 6) k_surface(Grid g, int n, const float4* __restrict__ pos,
-                                                 const float* __restrict__ rs, const int32_t* __restrict__ cs,
-                                                 int32_t* __restrict__ surface, float cone, float cos_cone,
-                                                 int min_nb, const unsigned int* __restrict__ rmax_bits,
-                                                 const float* __restrict__ mass, float merge_cut,
-                                                 float* __restrict__ ld_sum, int32_t* __restrict__ ld_cnt) {
+__device__ __forceinline__ bool in_cone(const SurfArgs& a, float3 xi, float3 xj, float reach, float3 c) {
+  float3 b = sub3(xj, xi);
+  if (sqrt_gt(dot3(b, b), reach)) return false;
+  b = m_normalize3<MM>(b);
+  const float d = dot3(b, c);
+  return d > a.cos_cone + 1e-5f ? true : (d < a.cos_cone - 1e-5f ? false : m_acos<MM>(d) <= a.cone);
+}
+
+// The vote over the stencil, the columns towards c first.  The vote is an OR
+// over the neighbours, so the order they are visited in is free: within a
+// column from the end c.z points to, so that an interior particle meets a
+// neighbour inside the cone early.
+template <int MM>
+__device__ __forceinline__ bool cone_vote(const SurfArgs& a, int i, float3 xi, int3 q, float ri, float R2, bool mixed,
+                                          float3 c) {
+  const Grid& g = a.g;
+  const int sx = c.x < 0.0f ? -1 : 1, sy = c.y < 0.0f ? -1 : 1;
+  const bool up = c.z > 0.0f;
+  // (64-bit cell coordinates: q saturates for positions far outside the grid)
+  const long long zl = max((long long)q.z - 1, 0LL), zh = min((long long)q.z + 1, (long long)g.nz - 1);
+  if (zl > zh) return false;
+  for (int o = 0; o < 9; ++o) {
+    const long long x = (long long)q.x + sx * kTowards[o][0], y = (long long)q.y + sy * kTowards[o][1];
+    if (x < 0 || x >= g.nx || y < 0 || y >= g.ny) continue;
+    const int k0 = (int)((x * g.ny + y) * g.nz + zl);
+    const int j0 = a.cs[k0], j1 = a.cs[k0 + (int)(zh - zl + 1)];
+    const int nch = (j1 - j0 + 31) >> 5;
+    for (int ch = 0; ch < nch; ++ch) {
+      const int c0 = j0 + 32 * (up ? nch - 1 - ch : ch);
+      unsigned mask = surface_chunk_mask(a.pos, c0, min(32, j1 - c0), i, xi, ri, R2, mixed, -1.0f);
+      while (mask) {
+        const int bit = up ? 31 - __clz(mask) : __ffs(mask) - 1;
+        mask &= ~(1u << bit);
+        const int j = c0 + bit;
+        if (in_cone<MM>(a, xi, f3(a.pos[j]), 2.0f * (ri + a.rs[j]), c)) return true;
+      }
+    }
+  }
+  return false;
+}
+
+constexpr int kSurfThreads = 256;
+
+template <int MM>
+__global__ void __launch_bounds__(kSurfThreads, 6) k_surface(SurfArgs a) {
+  const Grid g = a.g;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float3 xi = f3(pos[i]);
+  if (i >= a.n) return;
+  const float3 xi = f3(a.pos[i]);
   const int3 q = trunc_cell(g, xi);
-  const float ri = rs[i];
-  const float Rw = 2.0002f * (ri + __uint_as_float(*rmax_bits));
+  const float ri = a.rs[i];
+  const float wmax = __uint_as_float(*a.rmax_bits);
+  const float Rw = 2.0002f * (ri + wmax);
   const float R2 = Rw * Rw;
+  const bool mixed = __any_sync(__activemask(), wmax > kSurfMixed * ri);
   float3 cv = make_float3(0.f, 0.f, 0.f);
   unsigned nn = 0;
   // The merge scan's local density (merge_mark_gpu, Solver.cu:526-653): the
@@ -64,85 +148,198 @@ __global__ void __launch_bounds__(256, 6) k_surface(Grid g, int n, const float4*
   // candidate order.  Taken here when the prefilter reaches the merge
   // radius (its cut with the merge scan's own margin), so that the merge
   // scan only looks at candidates after i.
-  const bool ldc = ld_cnt && merge_cut * 1.0001f <= R2;
+  const bool ldc = a.ld_cnt && a.merge_cut * 1.0001f <= R2;
+  const float keep = ldc ? a.merge_cut * 1.0001f : -1.0f;
   float ld = 0.0f;
   int lc = 0;
   // Each stencil column is scanned in chunks of 32: the prefilter marks
   // the candidates that may lie within 2 (r_i + r_j) in a mask, and the
   // exact test and the sums run over the marked ones in candidate order.
   for_each_stencil_column(g, q, [&](int k0, int nc) {
-    const int j1 = cs[k0 + nc];
-    for (int c0 = cs[k0]; c0 < j1; c0 += 32) {
+    const int j1 = a.cs[k0 + nc];
+    for (int c0 = a.cs[k0]; c0 < j1; c0 += 32) {
       const int cn = min(32, j1 - c0);
-      unsigned mask = surface_chunk_mask(pos, c0, cn, i, xi, R2);
+      unsigned mask = surface_chunk_mask(a.pos, c0, cn, i, xi, ri, R2, mixed, keep);
       // the particle itself counts once, in the chunk that holds it
       const unsigned self = (unsigned)(i - c0);
       if (ldc && self < (unsigned)cn) mask |= 1u << self;
       while (mask) {
         const int j = c0 + __ffs(mask) - 1;
         mask &= mask - 1u;
-        const float3 d = sub3(xi, f3(pos[j]));
+        const float3 d = sub3(xi, f3(a.pos[j]));
         const float dd = dot3(d, d);
-        if (ldc && dd < merge_cut) {
-          ld += mass[j];
+        if (ldc && dd < a.merge_cut) {
+          ld += a.mass[j];
           ++lc;
         }
-        if (j == i || sqrt_gt(dd, 2.0f * (ri + rs[j]))) continue;
+        if (j == i || sqrt_gt(dd, 2.0f * (ri + a.rs[j]))) continue;
         cv = add3(cv, m_normalize3<MM>(d));
         ++nn;
       }
     }
   });
-  if (ld_cnt) {
-    ld_sum[i] = ld;
-    ld_cnt[i] = ldc ? lc : -1;
+  if (a.ld_cnt) {
+    a.ld_sum[i] = ld;
+    a.ld_cnt[i] = ldc ? lc : -1;
   }
-  if (nn <= (unsigned)min_nb) {
-    surface[i] = 1;
-    return;
+  bool vote = false;
+  if (nn > (unsigned)a.min_nb) vote = cone_vote<MM>(a, i, xi, q, ri, R2, mixed, m_normalize3<MM>(cv));
+  a.surface[i] = vote ? 0 : 1;
+}
+
+// The same with G lanes to a particle, for systems too small to fill the
+// chip with one thread each (k_sweep_group's scheme): the lanes test G
+// candidates at a time and list those within the prefilter's reach; G listed
+// ones at a time are tested exactly and added in candidate order, one lane
+// to a component; the vote runs over the list again, or, where it did not
+// hold all of them, over the stencil.
+//
+// Measured on a GB300 (same bits), thread against group: 51,000 particles of
+// the box scene 0.118 and 0.045 ms, 125,000 of the settled pile 0.44 and
+// 0.34 ms, 256,000 of a column 0.23 and 0.18 ms, 655,000 of a collapsed one
+// 0.98 and 0.91 ms, but 1,049,000 0.61 and 0.69 ms and 8.4 M 4.14 and
+// 5.39 ms: groups compute a particle's own values once a lane, and a chip
+// filled by threads gains nothing from them.
+constexpr int kSurfList = 128;
+constexpr int64_t kSurfGroupMax = 700000;
+
+template <int MM, int G>
+__global__ void __launch_bounds__(kSurfThreads) k_surface_group(SurfArgs a) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kGroups = kSurfThreads / G, kStep = 2 * G;
+  constexpr int kRow = 4 * G + (G < 32 ? 8 : 0);
+  __shared__ int32_t s_list[kGroups][kSurfList + kStep];
+  __shared__ int2 s_col[kGroups][9];
+  __shared__ float s_share[kGroups][kRow];
+  const Grid& g = a.g;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), grp = threadIdx.x / G;
+  const unsigned glt = (1u << gl) - 1u;
+  auto gballot = [&](bool p) {
+    const unsigned b = __ballot_sync(kAll, p);
+    return G == 32 ? b : (b >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u);
+  };
+  const int slot = blockIdx.x * kGroups + grp;
+  const bool act = slot < a.n;
+  const int i = act ? slot : a.n - 1;  // (groups past the end follow along and write nothing)
+  const float3 xi = f3(a.pos[i]);
+  const float ri = a.rs[i];
+  const float Rw = 2.0002f * (ri + __uint_as_float(*a.rmax_bits));
+  const float R2 = Rw * Rw;
+  const bool ldc = a.ld_cnt && a.merge_cut * 1.0001f <= R2;
+  const float keep = ldc ? a.merge_cut * 1.0001f : -1.0f;
+  const int3 q = trunc_cell(g, xi);
+  const long long zl = max((long long)q.z - 1, 0LL), zh = min((long long)q.z + 1, (long long)g.nz - 1);
+  for (int k = gl; k < 9; k += G) {
+    int2 col = make_int2(0, 0);
+    const long long x = (long long)q.x + k / 3 - 1, y = (long long)q.y + k % 3 - 1;
+    if (act && zl <= zh && x >= 0 && x < g.nx && y >= 0 && y < g.ny) {
+      const int k0 = (int)((x * g.ny + y) * g.nz + zl);
+      col = make_int2(a.cs[k0], a.cs[k0 + (int)(zh - zl + 1)]);
+    }
+    s_col[grp][k] = col;
+  }
+  __syncwarp();
+  float sum = 0.0f;  // component gl of the cover vector, or the density sum in lane 3
+  unsigned nn = 0;
+  int lc = 0, cnt = 0, col = 0, v = gl;
+  bool over = false;
+  for (;;) {
+    while (col < 9) {
+      const int2 js = s_col[grp][col];
+      bool full = false;
+      for (; __any_sync(kAll, js.x + v - gl < js.y); v += kStep) {
+        if ((full = __any_sync(kAll, cnt > kSurfList))) break;
+#pragma unroll
+        for (int u = 0; u < kStep; u += G) {
+          const int j = js.x + v + u;
+          bool hit = false;
+          if (j < js.y) {
+            hit = j == i ? ldc : surface_near(xi, ri, a.pos[j], keep);
+          }
+          const unsigned hb = gballot(hit);
+          if (hit) s_list[grp][cnt + __popc(hb & glt)] = j;
+          cnt += __popc(hb);
+        }
+      }
+      if (full) break;
+      v = gl;
+      ++col;
+    }
+    const bool done = col == 9;
+    const bool filled = cnt > kSurfList;
+    over |= filled;
+    __syncwarp();
+    const int n = done || filled ? cnt : 0;
+    for (int k0 = 0; __any_sync(kAll, k0 < n); k0 += G) {
+      bool nb = false, in = false;
+      float3 d = make_float3(0.f, 0.f, 0.f);
+      float m = 0.0f;
+      if (k0 + gl < n) {
+        const int j = s_list[grp][k0 + gl];
+        d = sub3(xi, f3(a.pos[j]));
+        const float dd = dot3(d, d);
+        in = ldc && dd < a.merge_cut;
+        if (in) m = a.mass[j];
+        nb = j != i && !sqrt_gt(dd, 2.0f * (ri + a.rs[j]));
+        if (nb) d = m_normalize3<MM>(d);
+      }
+      const unsigned nbb = gballot(nb), inb = gballot(in);
+      nn += __popc(nbb);
+      lc += __popc(inb);
+      if (nb) {
+        float* sh = &s_share[grp][__popc(nbb & glt)];
+        sh[0] = d.x;
+        sh[G] = d.y;
+        sh[2 * G] = d.z;
+      }
+      if (in) s_share[grp][3 * G + __popc(inb & glt)] = m;
+      __syncwarp();
+      if (gl < 4) {
+        const float* sh = &s_share[grp][gl * G];
+        const int num = __popc(gl == 3 ? inb : nbb);
+        for (int k = 0; k < num; ++k) sum += sh[k];
+      }
+      __syncwarp();
+    }
+    if (done) break;
+    if (filled) cnt = 0;
+  }
+  float3 cv;
+  cv.x = __shfl_sync(kAll, sum, 0, G);
+  cv.y = __shfl_sync(kAll, sum, 1, G);
+  cv.z = __shfl_sync(kAll, sum, 2, G);
+  if (act && a.ld_cnt) {
+    if (gl == 3) a.ld_sum[i] = sum;
+    if (gl == 0) a.ld_cnt[i] = ldc ? lc : -1;
   }
   const float3 c = m_normalize3<MM>(cv);
-  // The vote is an OR over the neighbours, so the order they are visited in
-  // is free: the stencil columns towards c first, and within a column from
-  // the end c.z points to, so that an interior particle meets a neighbour
-  // inside the cone early.  acos(d) <= cone is decided from d alone away
-  // from cos(cone) (the margin of 1e-5 on d is some 40 times the bound on
-  // acosf's error there and over the rounding of cos_cone, computed on the
-  // host); near it acos is evaluated.
-  const float d_in = cos_cone + 1e-5f, d_out = cos_cone - 1e-5f;
-  const int sx = c.x < 0.0f ? -1 : 1, sy = c.y < 0.0f ? -1 : 1;
-  const bool up = c.z > 0.0f;
-  // (64-bit cell coordinates: q saturates for positions far outside the grid)
-  const long long zl = max((long long)q.z - 1, 0LL), zh = min((long long)q.z + 1, (long long)g.nz - 1);
   bool vote = false;
-  if (zl <= zh) {
-    for (int o = 0; o < 9 && !vote; ++o) {
-      const long long x = (long long)q.x + sx * kTowards[o][0], y = (long long)q.y + sy * kTowards[o][1];
-      if (x < 0 || x >= g.nx || y < 0 || y >= g.ny) continue;
-      const int k0 = (int)((x * g.ny + y) * g.nz + zl);
-      const int j0 = cs[k0], j1 = cs[k0 + (int)(zh - zl + 1)];
-      const int nch = (j1 - j0 + 31) >> 5;
-      for (int ch = 0; ch < nch && !vote; ++ch) {
-        const int c0 = j0 + 32 * (up ? nch - 1 - ch : ch);
-        unsigned mask = surface_chunk_mask(pos, c0, min(32, j1 - c0), i, xi, R2);
-        while (mask) {
-          const int bit = up ? 31 - __clz(mask) : __ffs(mask) - 1;
-          mask &= ~(1u << bit);
-          const int j = c0 + bit;
-          float3 b = sub3(f3(pos[j]), xi);
-          if (sqrt_gt(dot3(b, b), 2.0f * (ri + rs[j]))) continue;
-          b = m_normalize3<MM>(b);
-          const float d = dot3(b, c);
-          const bool in = d > d_in ? true : (d < d_out ? false : m_acos<MM>(d) <= cone);
-          if (in) {
-            vote = true;
-            break;
-          }
-        }
+  bool open = act && nn > (unsigned)a.min_nb;
+  // the listed candidates, all of them unless the list overflowed
+  for (int k0 = 0; __any_sync(kAll, open && !over && k0 < cnt); k0 += G) {
+    bool in = false;
+    if (open && !over && k0 + gl < cnt) {
+      const int j = s_list[grp][k0 + gl];
+      in = j != i && in_cone<MM>(a, xi, f3(a.pos[j]), 2.0f * (ri + a.rs[j]), c);
+    }
+    if (gballot(in)) {
+      vote = true;
+      open = false;
+    }
+  }
+  for (int k = 0; k < 9 && __any_sync(kAll, open && over); ++k) {
+    const int2 js = s_col[grp][k];
+    for (int b = js.x; __any_sync(kAll, open && over && b < js.y); b += G) {
+      const int j = b + gl;
+      bool in = false;
+      if (open && over && j < js.y && j != i) in = in_cone<MM>(a, xi, f3(a.pos[j]), 2.0f * (ri + a.rs[j]), c);
+      if (gballot(in)) {
+        vote = true;
+        open = false;
       }
     }
   }
-  surface[i] = vote ? 0 : 1;
+  if (act && gl == 0) a.surface[i] = nn <= (unsigned)a.min_nb || !vote ? 1 : 0;
 }
 
 void merge_cuts(const gg_system* S, float& f_out, float& T_out);
@@ -151,13 +348,29 @@ gg_status surface(gg_system* S, cudaStream_t st) {
   if (S->n <= 0) return GG_OK;
   const int c = S->g.cur;
   prof_begin(S, PC_SURFACE, st);
-  auto kern = S->P.math_mode ? k_surface<1> : k_surface<0>;
-  float merge_f = 0.0f, merge_cut = 0.0f;
-  merge_cuts(S, merge_f, merge_cut);
-  kern<<<blocks_for(S->n, 256), 256, 0, st>>>(S->grid, (int)S->n, S->g.pos[c], S->g.rs[c], S->g.cell_start,
-                                               S->g.surface, S->P.surface_cone, std::cos(S->P.surface_cone),
-                                               S->P.surface_min_neighbors, &S->scal->rmax_bits, S->g.mass[c],
-                                               merge_cut, S->g.ld_sum, S->g.ld_cnt);
+  SurfArgs a;
+  a.g = S->grid;
+  a.n = (int)S->n;
+  a.pos = S->g.pos[c];
+  a.rs = S->g.rs[c];
+  a.cs = S->g.cell_start;
+  a.surface = S->g.surface;
+  a.cone = S->P.surface_cone;
+  a.cos_cone = std::cos(S->P.surface_cone);
+  a.min_nb = S->P.surface_min_neighbors;
+  a.rmax_bits = &S->scal->rmax_bits;
+  a.mass = S->g.mass[c];
+  float merge_f = 0.0f;
+  merge_cuts(S, merge_f, a.merge_cut);
+  a.ld_sum = S->g.ld_sum;
+  a.ld_cnt = S->g.ld_cnt;
+  if (S->n <= kSurfGroupMax) {
+    auto kern = S->P.math_mode ? k_surface_group<1, 8> : k_surface_group<0, 8>;
+    kern<<<blocks_for(S->n, kSurfThreads / 8), kSurfThreads, 0, st>>>(a);
+  } else {
+    auto kern = S->P.math_mode ? k_surface<1> : k_surface<0>;
+    kern<<<blocks_for(S->n, kSurfThreads), kSurfThreads, 0, st>>>(a);
+  }
   count_launches(S, 1);
   prof_end(S, PC_SURFACE, S->n, st);
   GG_CUDA(cudaGetLastError());
