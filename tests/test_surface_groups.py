@@ -46,3 +46,28 @@ def test_groups_match_oracle(n, spacing, heavy):
 @pytest.mark.parametrize("n", [700000, 700001])
 def test_both_sides_of_the_line_match_oracle(n):
     _check(n, 1.9, 0.1, radius=0.005)
+
+
+@pytest.mark.parametrize("reach", [0.035, 0.02])
+@pytest.mark.parametrize("n,spacing", [(1, 2.0), (9, 1.8), (257, 2.0), (4000, 1.9), (12000, 1.4)])
+def test_merge_scan_groups_match_oracle(n, spacing, reach):
+    """Partners and density of the merge: the radius inside the surface pass's
+    reach and beyond it, equal distances (an unjittered lattice)."""
+    r = workloads.REF_RADIUS
+    side = int(np.ceil(n ** (1 / 3)))
+    d = workloads.box_drop(2, substeps=8, adaptive=1)
+    s = spacing * r
+    p = workloads.lattice((side,) * 3, s, (0.2, 0.2, 0.2), 0.0 if spacing == 2.0 else 0.1 * s, 4)[:n]
+    masses = np.full(n, 0.5, np.float32)
+    d.update(particles=p, n_particles=n, masses=masses)
+    d["params"].math_mode, d["params"].min_merge_mass, d["params"].merge_radius = 1, 0.1, reach
+    d["params"].surface_dist_threshold = 0.0
+    g = gg.GranularSystem(**workloads.system_kwargs(d), masses=masses, device=0)
+    o = orc.OracleSystem(d, fp64=False)
+    for k in range(3):
+        for f in (gg.FIELD_REMOVE, gg.FIELD_MERGE, gg.FIELD_MERGE_VELOCITY, gg.FIELD_MASS, gg.FIELD_POS):
+            assert np.array_equal(g.read(f), o.read(f)), f"step {k}, field {f}"
+        g.step(1)
+        o.step(1)
+    g.close()
+    o.close()
