@@ -3,9 +3,10 @@
 // Replaces neighbor_search_{granular,boundary,upsampled}
 // (GranularSystem.cu:65-395) and the primitives of CUDAFunctions.cuh:54-107:
 //   cell key per particle  -> stable LSD radix sort of (key, index)
-//   -> one gather of every SoA field -> cell_start by count + exclusive scan.
+//   -> one gather of every SoA field -> cell_start from the sorted keys.
 // The sort is stable, as thrust::sort_by_key on int keys is, so the sorted
 // order is identical; it sorts only ceil(log2(C+1)) key bits.
+#include <algorithm>
 #include <mutex>
 #include <utility>
 
@@ -256,11 +257,155 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint32_t* 
   }
 }
 
+// ------------------------------------------------------------ short sort
+//
+// The same sort for inputs of at most kShortTiles tiles, in one launch for
+// the keys and one a digit (against four a digit): the launches and the gaps
+// between them were most of its time there.  A scatter block adds up the
+// tile histograms itself (256 threads, one a digit, at most 128 rows) where
+// the long sort scans them in three launches, and counts the next digit of
+// each item at the tile it lands in.  The counts rotate through three
+// tables: a pass reads one, adds to the next, and clears its row of the one
+// after that.  Measured on a GB300, hash and sort against the long sort:
+// 1,000 particles 18 and 50 us, 51,000 28 and 70 us, 125,000 50 and 95 us
+// (two digits, two and three); 200,000 on caller memory with the cell table
+// 51 and 97 us.  The rows that every block adds up set the limit.
+constexpr int kShortTiles = 128;
+constexpr int64_t short_max(int items) { return (int64_t)kShortTiles * kSortThreads * items; }
+constexpr int64_t kShortMax = short_max(16);  // 524,288; with 16 items a thread, fewer where fewer make as many tiles
+
+// A tile's keys and their first digits' counts.  kPacked: positions are
+// float[3], else float4.
+template <int kItems, bool kPacked>
+__global__ void __launch_bounds__(kSortThreads) k_hash_short(Grid g, const float* __restrict__ pos, int n,
+                                                             uint32_t* __restrict__ keys,
+                                                             uint32_t* __restrict__ keys_copy, int tiles,
+                                                             uint32_t* __restrict__ hist) {
+  __shared__ uint32_t h[256];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  const int base = blockIdx.x * kSortThreads * kItems;
+  const unsigned lt = lanemask_lt();
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    const int i = base + r * kSortThreads + threadIdx.x;
+    uint32_t d = 256u;
+    if (i < n) {
+      float3 p;
+      if (kPacked) p = make_float3(pos[3 * (int64_t)i], pos[3 * (int64_t)i + 1], pos[3 * (int64_t)i + 2]);
+      else p = f3(reinterpret_cast<const float4*>(pos)[i]);
+      const int3 c = floor_cell(g, p);
+      const uint32_t k = (uint32_t)cell_key(g, c.x, c.y, c.z);
+      keys[i] = k;
+      if (keys_copy) keys_copy[i] = k;
+      d = k & 255u;
+    }
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    if (i < n && (peers & lt) == 0) atomicAdd(&h[d], (uint32_t)__popc(peers));
+  }
+  __syncthreads();
+  const int row = blockIdx.x * 256 + threadIdx.x;
+  hist[row] = h[threadIdx.x];
+  hist[tiles * 256 + row] = 0;
+}
+
+// One digit: k_radix_scatter with the offsets worked out in the block.  vin
+// null: the values are the indices.
+template <int kItems>
+__global__ void __launch_bounds__(kSortThreads) k_scatter_short(const uint32_t* __restrict__ kin,
+                                                                const uint32_t* __restrict__ vin,
+                                                                uint32_t* __restrict__ kout,
+                                                                uint32_t* __restrict__ vout, int n, int pass,
+                                                                int tiles, uint32_t* __restrict__ hist, int last) {
+  constexpr int W = kSortThreads / 32, kTile = kSortThreads * kItems;
+  __shared__ uint32_t base_d[256];
+  __shared__ uint32_t wcnt[W][256];
+  const int t = threadIdx.x, warp = t >> 5, shift = 8 * pass;
+  const int base = blockIdx.x * kTile;
+  const int64_t table = (int64_t)tiles * 256;
+  const uint32_t* __restrict__ cur = hist + (pass % 3) * table;
+  uint32_t* next = hist + ((pass + 1) % 3) * table;
+  uint32_t k[kItems], v[kItems];
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    const int i = base + r * kSortThreads + t;
+    k[r] = i < n ? kin[i] : 0u;
+    v[r] = vin ? (i < n ? vin[i] : 0u) : (uint32_t)i;
+  }
+#pragma unroll
+  for (int w = 0; w < W; ++w) wcnt[w][t] = 0;
+  hist[((pass + 2) % 3) * table + blockIdx.x * 256 + t] = 0;
+  uint32_t before = 0, total = 0;
+#pragma unroll 16
+  for (int b = 0; b < tiles; ++b) {
+    const uint32_t c = cur[b * 256 + t];
+    if (b < (int)blockIdx.x) before += c;
+    total += c;
+  }
+  int all;
+  base_d[t] = before + (uint32_t)block_exclusive_scan<kSortThreads>((int)total, &all);
+  __syncthreads();
+  const unsigned lt = lanemask_lt();
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    const bool valid = base + r * kSortThreads + t < n;
+    const uint32_t d = (k[r] >> shift) & 255u;
+    const unsigned peers = __match_any_sync(0xffffffffu, valid ? d : 256u);
+    const bool leader = valid && (peers & lt) == 0;
+    const uint32_t cnt = (uint32_t)__popc(peers);
+    if (leader) wcnt[warp][d] = cnt;
+    __syncthreads();
+    if (valid) {
+      uint32_t dst = base_d[d] + (uint32_t)__popc(peers & lt);
+      for (int w = 0; w < warp; ++w) dst += wcnt[w][d];
+      kout[dst] = k[r];
+      vout[dst] = v[r];
+      if (!last) atomicAdd(&next[dst / kTile * 256 + ((k[r] >> (shift + 8)) & 255u)], 1u);
+    }
+    __syncthreads();
+    if (leader) {
+      atomicAdd(&base_d[d], cnt);
+      wcnt[warp][d] = 0;
+    }
+    __syncwarp();
+  }
+}
+
+template <int kItems, bool kPacked>
+static gg_status short_sort_items(const Grid& g, const float* pos, int n, SortScratch& s, uint32_t* keys_out,
+                                  uint32_t* perm_out, uint32_t* keys_unsorted_out, cudaStream_t st, gg_system* prof) {
+  const int tiles = (n + kSortThreads * kItems - 1) / (kSortThreads * kItems);
+  const int passes = (key_bits(g.C) + 7) / 8;
+  if (prof) prof_begin(prof, PC_HASH, st);
+  k_hash_short<kItems, kPacked><<<tiles, kSortThreads, 0, st>>>(g, pos, n, s.k[0], keys_unsorted_out, tiles, s.hist);
+  if (prof) prof_end(prof, PC_HASH, n, st);
+  if (prof) prof_begin(prof, PC_SORT, st);
+  for (int p = 0; p < passes; ++p) {
+    const bool last = p == passes - 1;
+    k_scatter_short<kItems><<<tiles, kSortThreads, 0, st>>>(
+        s.k[p & 1], p ? s.v[p & 1] : nullptr, last ? keys_out : s.k[(p & 1) ^ 1], last ? perm_out : s.v[(p & 1) ^ 1],
+        n, p, tiles, s.hist, last ? 1 : 0);
+  }
+  if (prof) prof_end(prof, PC_SORT, n, st);
+  if (s.counter) *s.counter += 1 + passes;
+  GG_CUDA(cudaGetLastError());
+  return GG_OK;
+}
+
+template <bool kPacked>
+static gg_status short_sort(const Grid& g, const float* pos, int64_t n, SortScratch& s, uint32_t* keys_out,
+                            uint32_t* perm_out, uint32_t* keys_unsorted_out, cudaStream_t st, gg_system* prof) {
+  auto sort = n <= short_max(4)   ? short_sort_items<4, kPacked>
+              : n <= short_max(8) ? short_sort_items<8, kPacked>
+                                  : short_sort_items<16, kPacked>;
+  return sort(g, pos, (int)n, s, keys_out, perm_out, keys_unsorted_out, st, prof);
+}
+
 gg_status sort_scratch_alloc(SortScratch& s, int64_t capacity) {
   if (capacity < 1) capacity = 1;
   s.capacity = capacity;
   const int64_t tiles = (capacity + kSortTile - 1) / kSortTile;
-  s.hist_entries = tiles * 256;
+  s.hist_entries = std::max<int64_t>(tiles, 3 * kShortTiles) * 256;
   // scan blocks must cover the largest scanned array: hist, cell table, particles
   s.scan_block_entries = kScanMaxBlocks;
   for (int i = 0; i < 2; ++i) {
@@ -285,10 +430,10 @@ void sort_scratch_free(SortScratch& s) {
 }
 
 // Stable LSD sort of the (key, value) pairs held in s.k[0], s.v[0]; the
-// last pass writes keys_out / perm_out.  hist0_ready: s.hist already holds
-// the first digit's tile histogram (counted by the hash kernel).
+// last pass writes keys_out / perm_out.  s.hist already holds the first
+// digit's tile histogram (counted by the hash kernel).
 static gg_status radix_sort_pairs(const Grid& g, int64_t n, SortScratch& s, uint32_t* keys_out, uint32_t* perm_out,
-                                  cudaStream_t st, bool hist0_ready) {
+                                  cudaStream_t st) {
   const int nn = (int)n;
   const int bits = key_bits(g.C);
   const int passes = (bits + 7) / 8;
@@ -299,7 +444,7 @@ static gg_status radix_sort_pairs(const Grid& g, int64_t n, SortScratch& s, uint
     const bool last = p == passes - 1;
     uint32_t* ko = last ? keys_out : s.k[src ^ 1];
     uint32_t* vo = last ? perm_out : s.v[src ^ 1];
-    if (p > 0 || !hist0_ready) {
+    if (p > 0) {
       k_radix_hist<<<tiles, kSortThreads, 0, st>>>(s.k[src], nn, shift, tiles, s.hist);
       if (s.counter) *s.counter += 1;
     }
@@ -320,6 +465,9 @@ gg_status grid_sort(const Grid& g, const float4* pos, int64_t n, SortScratch& s,
     set_error("grid_sort: more elements than the sort scratch holds");
     return GG_ERR_INVALID_ARGUMENT;
   }
+  if (n <= kShortMax)
+    return short_sort<false>(g, reinterpret_cast<const float*>(pos), n, s, keys_out, perm_out, keys_unsorted_out, st,
+                             prof);
   const int nn = (int)n;
   if (prof) prof_begin(prof, PC_HASH, st);
   const int tiles = (int)((n + kSortTile - 1) / kSortTile);
@@ -327,34 +475,107 @@ gg_status grid_sort(const Grid& g, const float4* pos, int64_t n, SortScratch& s,
   if (s.counter) *s.counter += 1;
   if (prof) prof_end(prof, PC_HASH, n, st);
   if (prof) prof_begin(prof, PC_SORT, st);
-  gg_status rc = radix_sort_pairs(g, n, s, keys_out, perm_out, st, true);
+  gg_status rc = radix_sort_pairs(g, n, s, keys_out, perm_out, st);
   if (prof) prof_end(prof, PC_SORT, n, st);
   return rc;
 }
 
 // ------------------------------------------------------------ cell start
 
-// countingInCell_CUDA (CUDAFunctions.cuh:54-61) on the sorted keys, one
-// atomic per run of equal keys in a warp.
-__global__ void k_count_cells(const uint32_t* __restrict__ keys, int n, int32_t* __restrict__ counts) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t k = i < n ? keys[i] : 0xffffffffu;
-  const unsigned peers = __match_any_sync(0xffffffffu, k);
-  if (i < n && __popc(peers & lanemask_lt()) == 0) atomicAdd(&counts[k], __popc(peers));
+// countingInCell_CUDA (CUDAFunctions.cuh:54-61) and its scan, from the
+// sorted keys in one launch.  The cells 0 .. C and the sorted keys form one
+// merged order, a cell before the keys that are its own or later; cell c's
+// start is the number of keys before it.  Key k has k keys and keys[k] + 1
+// cells before it, so its place is k + keys[k] + 1, and a warp finds the
+// kCellWindow consecutive places that are its own by searching the keys:
+// however the particles crowd, a warp has no more than that many.  It notes
+// the first particle of each cell that has one, and fills the others from
+// the right with the next cell's first.  (Clearing, counting with atomics
+// and scanning took five launches: 24 us for 1,000 particles in 15,000 cells
+// against 10 us here, 24 and 16 us for 125,000 in 247,000, 54 and 28 us for
+// 655,000 and 77 and 71 us for 8.4 M in 3.8 M.  The same by windows of 256
+// cells took 919 us on the last one, whose out-of-grid cell is crowded.)
+constexpr int kCellWindow = 512, kCellWarps = 8;
+
+// The number of keys whose place is before `place`, by all lanes of a warp:
+// 32 probes a step.
+__device__ __forceinline__ int keys_before(const uint32_t* __restrict__ keys, int n, int64_t place) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, len = n;
+  while (len > 32) {
+    const int step = (len + 31) >> 5;
+    const int at = lane * step + step - 1;  // the last of this lane's part
+    const unsigned less = __ballot_sync(0xffffffffu, at < len && (int64_t)(lo + at) + keys[lo + at] + 1 < place);
+    const int skip = __popc(less) * step;   // (parts wholly before, which come first)
+    lo += skip;
+    len = min(step, len - skip);
+  }
+  return lo + __popc(__ballot_sync(0xffffffffu, lane < len && (int64_t)(lo + lane) + keys[lo + lane] + 1 < place));
+}
+
+__global__ void __launch_bounds__(32 * kCellWarps) k_cell_start(const uint32_t* __restrict__ keys, int n, int entries,
+                                                                int32_t* __restrict__ cell_start) {
+  __shared__ int s_first[kCellWarps][kCellWindow];
+  __shared__ int s_key[kCellWarps + 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t place = ((int64_t)blockIdx.x * kCellWarps + w) * kCellWindow;
+  const int mine = keys_before(keys, n, place);
+  const int end = w == kCellWarps - 1 ? keys_before(keys, n, place + kCellWindow) : 0;
+  if (lane == 0) {
+    s_key[w] = mine;
+    if (w == kCellWarps - 1) s_key[kCellWarps] = end;
+  }
+  __syncthreads();
+  const int k0 = s_key[w], k1 = s_key[w + 1];
+  const int64_t c0 = place - k0;  // the cells c0 .. c0 + own - 1 are this warp's
+  const int own = (int)min(place + kCellWindow - k1, (int64_t)entries) - (int)min(c0, (int64_t)entries);
+  if (own <= 0) return;
+  int* first = s_first[w];
+#pragma unroll
+  for (int k = lane; k < kCellWindow; k += 32) first[k] = k1;
+  __syncwarp();
+#pragma unroll 4
+  for (int p = k0 + lane; p < k1; p += 32) {
+    const int64_t c = (int64_t)keys[p] - c0;
+    if (c >= 0 && c < own && (p == k0 || keys[p - 1] != keys[p])) first[c] = p;
+  }
+  __syncwarp();
+  // a lane's consecutive cells from the right, then the lanes' firsts
+  constexpr int kOwn = kCellWindow / 32;
+  int v[kOwn];
+#pragma unroll
+  for (int k = 0; k < kOwn; ++k) v[k] = first[lane * kOwn + k];
+#pragma unroll
+  for (int k = kOwn - 2; k >= 0; --k) v[k] = min(v[k], v[k + 1]);
+  int rest = v[0];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_down_sync(0xffffffffu, rest, o);
+    if (lane + o < 32) rest = min(rest, y);
+  }
+  int right = __shfl_down_sync(0xffffffffu, rest, 1);
+  if (lane == 31) right = k1;
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < kOwn; ++k) first[lane * kOwn + k] = min(v[k], right);
+  __syncwarp();
+  for (int k = lane; k < own; k += 32) cell_start[c0 + k] = first[k];
 }
 
 gg_status cell_start_build(const Grid& g, const uint32_t* sorted_keys, int64_t n, int32_t* cell_start,
                            SortScratch& s, cudaStream_t st, gg_system* prof) {
   if (prof) prof_begin(prof, PC_CELLSTART, st);
-  GG_CUDA(cudaMemsetAsync(cell_start, 0, sizeof(int32_t) * ((int64_t)g.C + 1), st));
+  const int entries = g.C + 1;
   if (n > 0) {
-    k_count_cells<<<blocks_for(n, 256), 256, 0, st>>>(sorted_keys, (int)n, cell_start);
+    k_cell_start<<<blocks_for(n + entries, kCellWindow * kCellWarps), 32 * kCellWarps, 0, st>>>(
+        sorted_keys, (int)n, entries, cell_start);
     if (s.counter) *s.counter += 1;
+  } else {
+    GG_CUDA(cudaMemsetAsync(cell_start, 0, sizeof(int32_t) * (size_t)entries, st));
   }
-  gg_status rc = exclusive_scan(cell_start, cell_start, (int64_t)g.C + 1, s, st, nullptr);
-  if (prof) prof_end(prof, PC_CELLSTART, (int64_t)g.C + 1, st);
+  if (prof) prof_end(prof, PC_CELLSTART, entries, st);
   GG_CUDA(cudaGetLastError());
-  return rc;
+  return GG_OK;
 }
 
 // --------------------------------------------------------------- reorder
@@ -454,32 +675,19 @@ gg_status reorder_upsampled(gg_system* S, const uint32_t* perm, cudaStream_t st)
 // code hosted inside an engine or framework that owns every device
 // allocation, or a loop that must not allocate once it is running.  The
 // caller passes device buffers for the positions and for every output; the
-// sort's scratch (two key/value ping-pong buffers, the per-tile digit
-// histograms and the scan's block sums) lives in the file-scope array below,
-// sized for at most kNoAllocMaxParticles particles and kNoAllocMaxCells
-// cells.  Every GPU that loads this library holds that array (about 4.1 MiB)
-// until the process exits.
+// sort's scratch (two key/value ping-pong buffers and three tables of the
+// per-tile digit counts) lives in the file-scope array below, sized for at
+// most kNoAllocMaxParticles particles.  Every GPU that loads this library
+// holds that array (about 4.4 MiB) until the process exits.
 
 constexpr int64_t kNoAllocMaxParticles = 1 << 18;
 constexpr int64_t kNoAllocMaxCells = 1 << 24;
-constexpr int64_t kNoAllocTiles = (kNoAllocMaxParticles + kSortTile - 1) / kSortTile;
+static_assert(kNoAllocMaxParticles <= kShortMax, "the short sort reaches the limit");
 constexpr size_t kNoAllocPairWords = 4 * (size_t)kNoAllocMaxParticles;   // k0, k1, v0, v1
-constexpr size_t kNoAllocHistWords = 256 * (size_t)kNoAllocTiles;
-constexpr size_t kNoAllocScanWords = (size_t)kScanMaxBlocks;
-constexpr size_t kNoAllocWords = kNoAllocPairWords + kNoAllocHistWords + kNoAllocScanWords;
+constexpr size_t kNoAllocHistWords = 3 * 256 * (size_t)kShortTiles;
+constexpr size_t kNoAllocWords = kNoAllocPairWords + kNoAllocHistWords;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
-
-// mapParticles2Cells_CUDA over packed float[3] positions (12-byte stride).
-__global__ void k_hash3(Grid g, const float* __restrict__ pos3, int n, uint32_t* __restrict__ keys,
-                        uint32_t* __restrict__ vals) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float3 p = make_float3(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2]);
-  const int3 c = floor_cell(g, p);
-  keys[i] = (uint32_t)cell_key(g, c.x, c.y, c.z);
-  vals[i] = (uint32_t)i;
-}
 
 namespace {
 // Saves the calling thread's current device and restores it on scope exit.
@@ -551,10 +759,8 @@ extern "C" gg_status gg_grid_build_noalloc(int32_t device, const float* d_pos, i
     s.v[0] = base + 2 * kNoAllocMaxParticles;
     s.v[1] = base + 3 * kNoAllocMaxParticles;
     s.hist = base + kNoAllocPairWords;
-    s.scan_blocks = (int32_t*)(base + kNoAllocPairWords + kNoAllocHistWords);
     s.capacity = kNoAllocMaxParticles;
     s.hist_entries = (int64_t)kNoAllocHistWords;
-    s.scan_block_entries = (int64_t)kNoAllocScanWords;
     Grid g;
     g.L = cell_length;
     g.nx = cell_size[0];
@@ -563,14 +769,11 @@ extern "C" gg_status gg_grid_build_noalloc(int32_t device, const float* d_pos, i
     g.C = (int)C;
     cudaStream_t st = (cudaStream_t)stream;
     if (n > 0) {
-      k_hash3<<<blocks_for(n, 256), 256, 0, st>>>(g, d_pos, (int)n, s.k[0], s.v[0]);
-      GG_CUDA(cudaGetLastError());
-      rc = radix_sort_pairs(g, n, s, d_sorted_keys, d_perm, st, false);
+      rc = short_sort<true>(g, d_pos, n, s, d_sorted_keys, d_perm, nullptr, st, nullptr);
       if (rc != GG_OK) return rc;
     }
-    // cell_start_build clears the caller's table (the counts start at zero)
-    // before counting; the histograms and block sums in the scratch are
-    // fully written before they are read, so they need no clearing.
+    // (the sort's tables are written before they are read, so what the last
+    // call left there needs no clearing)
     return cell_start_build(g, d_sorted_keys, n, d_cell_start, s, st, nullptr);
   } catch (...) {
     set_error("gg_grid_build_noalloc: internal error");

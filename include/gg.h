@@ -460,7 +460,7 @@ void gg_grid_destroy(gg_grid* g);
  * The results equal gg_grid_build's.  The sort's scratch memory is a fixed
  * array inside the library, sized for at most 262,144 particles and
  * 16,777,216 cells; larger inputs return GG_ERR_CAPACITY with a message.
- * Every GPU that loads the library keeps that array (about 4.1 MiB) until
+ * Every GPU that loads the library keeps that array (about 4.4 MiB) until
  * the process exits.
  *   - The first call on a device looks up the array's device address; make
  *     that first call before any stream capture on that device.
