@@ -191,6 +191,45 @@ __host__ __device__ __forceinline__ float residual_mean(double sum, unsigned int
   return count ? (float)(sum / (double)count) : 0.0f;
 }
 
+// Programmatic dependent launch, for the chains of short kernels: a kernel
+// launched by launch_chained is set up on the chip while the one before it
+// in the stream ends, and its first pdl_wait returns once that one (and so
+// every one before it) has completed and its writes are visible.  Every
+// kernel launched this way calls pdl_wait before it touches memory, and
+// derives its addresses from the value that comes back (the thread index
+// that it is given), so that no load can be moved ahead of the wait; and none
+// of its loads takes the read-only path (no __restrict__ const pointer),
+// which may return what the cache held before.  Measured on a GB300 with the
+// clears and copies between the kernels folded into them: a frame of 4
+// substeps of 1,000 particles 776 to 486 us, a warm-started substep of 76
+// sweeps 6.1 to 4.3 ms, a grid build of 200,000 points 51 to 41 us.  (Letting the next kernel's
+// blocks in earlier, with an explicit trigger, measured slower: they take
+// the place of the blocks still to run.)
+__device__ __forceinline__ unsigned int pdl_wait(unsigned int tid) {
+  unsigned int r;
+  asm volatile(
+      "griddepcontrol.wait;\n\t"
+      "mov.u32 %0, %1;"
+      : "=r"(r)
+      : "r"(tid)
+      : "memory");
+  return r;
+}
+
+template <class... Params, class... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), int blocks, int threads, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 __device__ __forceinline__ unsigned int lanemask_lt() {
   unsigned int m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -118,7 +118,9 @@ struct Granular {
   int4* nl_meta = nullptr;    // query cell at list build, entry count (-1 = overflow)
   float* nl_acc = nullptr;    // displacement bound summed since the particle's list build
   int32_t* nl_queue = nullptr; // particles whose list is rebuilt in this sweep
-  uint32_t* cell_inc = nullptr; // per cell (C+1): max |x* increment| of its particles in the last sweep (float bits)
+  // per cell (C+1): max |x* increment| of its particles in a sweep (float
+  // bits); the sweeps take turns, the next one reading the last one's
+  uint32_t* cell_inc[2] = {nullptr, nullptr};
   float* ld_sum = nullptr;       // surface pass: mass within the merge radius, in candidate order
   int32_t* ld_cnt = nullptr;     // and the count (-1: not computed there)
   // grid
@@ -308,6 +310,7 @@ gg_status window_table(gg_system* S, cudaStream_t st);
 // res (only where sweep_sums_residual holds): the sweep also sums the
 // penetrations at x* there, and does nothing once scal->res_done is set.
 gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res = nullptr);
+bool sweep_lists(const gg_system* S);  // the sweep keeps contact lists
 bool sweep_sums_residual(const gg_system* S);
 // last: write the constraint counts (the substep's last sweep, or every
 // sweep of the residual mode); more: another sweep may follow, so record the

@@ -277,18 +277,19 @@ constexpr int64_t kShortMax = short_max(16);  // 524,288; with 16 items a thread
 // A tile's keys and their first digits' counts.  kPacked: positions are
 // float[3], else float4.
 template <int kItems, bool kPacked>
-__global__ void __launch_bounds__(kSortThreads) k_hash_short(Grid g, const float* __restrict__ pos, int n,
-                                                             uint32_t* __restrict__ keys,
-                                                             uint32_t* __restrict__ keys_copy, int tiles,
-                                                             uint32_t* __restrict__ hist) {
+__global__ void __launch_bounds__(kSortThreads) k_hash_short(Grid g, const float* pos, int n,
+                                                             uint32_t* keys,
+                                                             uint32_t* keys_copy, int tiles,
+                                                             uint32_t* hist) {
   __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
+  const int t = (int)pdl_wait(threadIdx.x);
+  h[t] = 0;
   __syncthreads();
   const int base = blockIdx.x * kSortThreads * kItems;
   const unsigned lt = lanemask_lt();
 #pragma unroll
   for (int r = 0; r < kItems; ++r) {
-    const int i = base + r * kSortThreads + threadIdx.x;
+    const int i = base + r * kSortThreads + t;
     uint32_t d = 256u;
     if (i < n) {
       float3 p;
@@ -304,26 +305,26 @@ __global__ void __launch_bounds__(kSortThreads) k_hash_short(Grid g, const float
     if (i < n && (peers & lt) == 0) atomicAdd(&h[d], (uint32_t)__popc(peers));
   }
   __syncthreads();
-  const int row = blockIdx.x * 256 + threadIdx.x;
-  hist[row] = h[threadIdx.x];
+  const int row = blockIdx.x * 256 + t;
+  hist[row] = h[t];
   hist[tiles * 256 + row] = 0;
 }
 
 // One digit: k_radix_scatter with the offsets worked out in the block.  vin
 // null: the values are the indices.
 template <int kItems>
-__global__ void __launch_bounds__(kSortThreads) k_scatter_short(const uint32_t* __restrict__ kin,
-                                                                const uint32_t* __restrict__ vin,
-                                                                uint32_t* __restrict__ kout,
-                                                                uint32_t* __restrict__ vout, int n, int pass,
-                                                                int tiles, uint32_t* __restrict__ hist, int last) {
+__global__ void __launch_bounds__(kSortThreads) k_scatter_short(const uint32_t* kin,
+                                                                const uint32_t* vin,
+                                                                uint32_t* kout,
+                                                                uint32_t* vout, int n, int pass,
+                                                                int tiles, uint32_t* hist, int last) {
   constexpr int W = kSortThreads / 32, kTile = kSortThreads * kItems;
   __shared__ uint32_t base_d[256];
   __shared__ uint32_t wcnt[W][256];
-  const int t = threadIdx.x, warp = t >> 5, shift = 8 * pass;
+  const int t = (int)pdl_wait(threadIdx.x), warp = t >> 5, shift = 8 * pass;
   const int base = blockIdx.x * kTile;
   const int64_t table = (int64_t)tiles * 256;
-  const uint32_t* __restrict__ cur = hist + (pass % 3) * table;
+  const uint32_t* cur = hist + (pass % 3) * table;
   uint32_t* next = hist + ((pass + 1) % 3) * table;
   uint32_t k[kItems], v[kItems];
 #pragma unroll
@@ -377,14 +378,15 @@ static gg_status short_sort_items(const Grid& g, const float* pos, int n, SortSc
   const int tiles = (n + kSortThreads * kItems - 1) / (kSortThreads * kItems);
   const int passes = (key_bits(g.C) + 7) / 8;
   if (prof) prof_begin(prof, PC_HASH, st);
-  k_hash_short<kItems, kPacked><<<tiles, kSortThreads, 0, st>>>(g, pos, n, s.k[0], keys_unsorted_out, tiles, s.hist);
+  GG_CUDA(launch_chained(k_hash_short<kItems, kPacked>, tiles, kSortThreads, st, g, pos, n, s.k[0], keys_unsorted_out,
+                         tiles, s.hist));
   if (prof) prof_end(prof, PC_HASH, n, st);
   if (prof) prof_begin(prof, PC_SORT, st);
   for (int p = 0; p < passes; ++p) {
     const bool last = p == passes - 1;
-    k_scatter_short<kItems><<<tiles, kSortThreads, 0, st>>>(
-        s.k[p & 1], p ? s.v[p & 1] : nullptr, last ? keys_out : s.k[(p & 1) ^ 1], last ? perm_out : s.v[(p & 1) ^ 1],
-        n, p, tiles, s.hist, last ? 1 : 0);
+    GG_CUDA(launch_chained(k_scatter_short<kItems>, tiles, kSortThreads, st, s.k[p & 1], p ? s.v[p & 1] : nullptr,
+                           last ? keys_out : s.k[(p & 1) ^ 1], last ? perm_out : s.v[(p & 1) ^ 1], n, p, tiles, s.hist,
+                           last ? 1 : 0));
   }
   if (prof) prof_end(prof, PC_SORT, n, st);
   if (s.counter) *s.counter += 1 + passes;
@@ -499,8 +501,7 @@ constexpr int kCellWindow = 512, kCellWarps = 8;
 
 // The number of keys whose place is before `place`, by all lanes of a warp:
 // 32 probes a step.
-__device__ __forceinline__ int keys_before(const uint32_t* __restrict__ keys, int n, int64_t place) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ int keys_before(const uint32_t* keys, int n, int64_t place, int lane) {
   int lo = 0, len = n;
   while (len > 32) {
     const int step = (len + 31) >> 5;
@@ -513,14 +514,14 @@ __device__ __forceinline__ int keys_before(const uint32_t* __restrict__ keys, in
   return lo + __popc(__ballot_sync(0xffffffffu, lane < len && (int64_t)(lo + lane) + keys[lo + lane] + 1 < place));
 }
 
-__global__ void __launch_bounds__(32 * kCellWarps) k_cell_start(const uint32_t* __restrict__ keys, int n, int entries,
-                                                                int32_t* __restrict__ cell_start) {
+__global__ void __launch_bounds__(32 * kCellWarps) k_cell_start(const uint32_t* keys, int n, int entries,
+                                                                int32_t* cell_start) {
   __shared__ int s_first[kCellWarps][kCellWindow];
   __shared__ int s_key[kCellWarps + 1];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int t = (int)pdl_wait(threadIdx.x), lane = t & 31, w = t >> 5;
   const int64_t place = ((int64_t)blockIdx.x * kCellWarps + w) * kCellWindow;
-  const int mine = keys_before(keys, n, place);
-  const int end = w == kCellWarps - 1 ? keys_before(keys, n, place + kCellWindow) : 0;
+  const int mine = keys_before(keys, n, place, lane);
+  const int end = w == kCellWarps - 1 ? keys_before(keys, n, place + kCellWindow, lane) : 0;
   if (lane == 0) {
     s_key[w] = mine;
     if (w == kCellWarps - 1) s_key[kCellWarps] = end;
@@ -567,8 +568,8 @@ gg_status cell_start_build(const Grid& g, const uint32_t* sorted_keys, int64_t n
   if (prof) prof_begin(prof, PC_CELLSTART, st);
   const int entries = g.C + 1;
   if (n > 0) {
-    k_cell_start<<<blocks_for(n + entries, kCellWindow * kCellWarps), 32 * kCellWarps, 0, st>>>(
-        sorted_keys, (int)n, entries, cell_start);
+    GG_CUDA(launch_chained(k_cell_start, blocks_for(n + entries, kCellWindow * kCellWarps), 32 * kCellWarps, st,
+                           sorted_keys, (int)n, entries, cell_start));
     if (s.counter) *s.counter += 1;
   } else {
     GG_CUDA(cudaMemsetAsync(cell_start, 0, sizeof(int32_t) * (size_t)entries, st));
@@ -583,18 +584,20 @@ gg_status cell_start_build(const Grid& g, const uint32_t* sorted_keys, int64_t n
 // The gathers of GranularSystem.cu:97-135 for every permuted field in one
 // pass.  adaptive_last_step and merge_velocity are not permuted, as in the
 // reference.
-__global__ void k_reorder_granular(int n, const uint32_t* __restrict__ perm,
-                                   const float4* __restrict__ pos_in, float4* __restrict__ pos_out,
-                                   const float4* __restrict__ vel_in, float4* __restrict__ vel_out,
-                                   const float* __restrict__ mass_in, float* __restrict__ mass_out,
-                                   const float* __restrict__ rs_in, float* __restrict__ rs_out,
-                                   const int32_t* __restrict__ units_in, int32_t* __restrict__ units_out,
-                                   const float* __restrict__ merge_in, float* __restrict__ merge_out,
-                                   const int32_t* __restrict__ mu_in, int32_t* __restrict__ mu_out,
-                                   const int32_t* __restrict__ mc_in, int32_t* __restrict__ mc_out,
-                                   const int32_t* __restrict__ rm_in, int32_t* __restrict__ rm_out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_reorder_granular(int n, const uint32_t* perm,
+                                   const float4* pos_in, float4* pos_out,
+                                   const float4* vel_in, float4* vel_out,
+                                   const float* mass_in, float* mass_out,
+                                   const float* rs_in, float* rs_out,
+                                   const int32_t* units_in, int32_t* units_out,
+                                   const float* merge_in, float* merge_out,
+                                   const int32_t* mu_in, int32_t* mu_out,
+                                   const int32_t* mc_in, int32_t* mc_out,
+                                   const int32_t* rm_in, int32_t* rm_out,
+                                   const int32_t* als_in, int32_t* als_out) {
+  const int p = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   if (p >= n) return;
+  als_out[p] = als_in[p];  // stays where it is
   const uint32_t s = perm[p];
   pos_out[p] = pos_in[s];
   vel_out[p] = vel_in[s];
@@ -612,13 +615,11 @@ gg_status reorder_granular(gg_system* S, cudaStream_t st) {
   Granular& G = S->g;
   const int a = G.cur, b = G.cur ^ 1;
   prof_begin(S, PC_REORDER, st);
-  k_reorder_granular<<<blocks_for(S->n, 256), 256, 0, st>>>(
-      (int)S->n, G.perm, G.pos[a], G.pos[b], G.vel[a], G.vel[b], G.mass[a], G.mass[b], G.rs[a], G.rs[b],
+  GG_CUDA(launch_chained(
+      k_reorder_granular, blocks_for(S->n, 256), 256, st, (int)S->n, G.perm, G.pos[a], G.pos[b], G.vel[a], G.vel[b], G.mass[a], G.mass[b], G.rs[a], G.rs[b],
       G.units[a], G.units[b], G.merge[a], G.merge[b], G.merge_units[a], G.merge_units[b],
-      G.merge_count[a], G.merge_count[b], G.remove[a], G.remove[b]);
+      G.merge_count[a], G.merge_count[b], G.remove[a], G.remove[b], G.als[a], G.als[b]));
   count_launches(S, 1);
-  // adaptive_last_step stays where it is: copy it into the new live buffer
-  GG_CUDA(cudaMemcpyAsync(G.als[b], G.als[a], sizeof(int32_t) * S->n, cudaMemcpyDeviceToDevice, st));
   prof_end(S, PC_REORDER, S->n, st);
   G.cur = b;
   GG_CUDA(cudaGetLastError());

@@ -39,14 +39,17 @@ gg_status radii_all(gg_system* S, cudaStream_t st) {
 
 // v += dt*G (Solver.cu:125-131); x* = x + dt*v (:133-160);
 // scaled mass m*exp(-y) (:162-191) kept as its reciprocal (:317).
-// Also the pruning bounds: max contact radius and max |x* - x|.
+// Also the pruning bounds: max contact radius and max |x* - x|; with the
+// Coulomb law (pn) the substep's normal corrections start at zero.
 template <int MM>
-__global__ void k_predict(int n, const float4* __restrict__ pos, const float4* __restrict__ vel,
-                          const float* __restrict__ mass, float4* __restrict__ xs,
-                          float* __restrict__ inv_m, float dt, float3 dv, DevScalars* scal) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_predict(int n, const float4* pos, const float4* vel,
+                          const float* mass, float4* xs,
+                          float* inv_m, float dt, float3 dv, DevScalars* scal,
+                          float* pn) {
+  const int i = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   unsigned int rbits = 0, dbits = 0;
   if (i < n) {
+    if (pn) pn[i] = 0.0f;
     const float4 p = pos[i];
     const float4 v4 = vel[i];
     const float3 v = add3(f3(v4), dv);
@@ -69,8 +72,8 @@ gg_status predict(gg_system* S, cudaStream_t st) {
   prof_begin(S, PC_PREDICT, st);
   auto kern = S->P.math_mode ? k_predict<1> : k_predict<0>;
   const int tp = S->tune.predict_threads;
-  kern<<<blocks_for(S->n, tp), tp, 0, st>>>((int)S->n, S->g.pos[c], S->g.vel[c], S->g.mass[c], S->g.xs,
-                                                   S->g.inv_m, dt, dv, S->scal);
+  GG_CUDA(launch_chained(kern, blocks_for(S->n, tp), tp, st, (int)S->n, S->g.pos[c], S->g.vel[c], S->g.mass[c],
+                         S->g.xs, S->g.inv_m, dt, dv, S->scal, S->P.contact_law == 1 ? S->g.pn : nullptr));
   count_launches(S, 1);
   prof_end(S, PC_PREDICT, S->n, st);
   GG_CUDA(cudaGetLastError());
@@ -88,12 +91,12 @@ struct PlaneArgs {
   // slab floor(x / W)) and, when given, Coulomb coefficients per scene
   int n_scenes;
   float scene_w, scene_inv_w;
-  const float2* __restrict__ scene_mu;
+  const float2* scene_mu;
 };
 
 // Residual mode: the sweep's penetrations and the target they are held to.
 struct ResidualArgs {
-  const ResidualSlot* __restrict__ res;  // null: apply always
+  const volatile ResidualSlot* res;  // null: apply always
   volatile int* done;
   float target;
   int it;
@@ -114,14 +117,14 @@ struct ResidualArgs {
 // corrections and the wall projections), else cut to mu_kinetic times it.
 // In a batch of scenes the walls are in each scene's own coordinates and
 // the coefficients those of the particle's scene.
-__global__ void __launch_bounds__(256) k_apply(int n, float4* __restrict__ xs, float4* __restrict__ pos,
-                        const float4* __restrict__ delta, int32_t* __restrict__ s_extra,
-                        int32_t* __restrict__ ncon, int32_t* __restrict__ contacts, int stab, int last,
-                        unsigned int* __restrict__ inc_bits, unsigned int* __restrict__ inc_norm_bits,
-                        const uint32_t* __restrict__ keys,
-                        uint32_t* __restrict__ cell_inc, int C, int nz, UDiv div_z, PlaneArgs pa,
-                        const float4* __restrict__ fdelta, float* __restrict__ pn, ResidualArgs ra) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_apply(int n, float4* xs, float4* pos,
+                        const float4* delta, int32_t* s_extra,
+                        int32_t* ncon, int32_t* contacts, int stab, int last,
+                        unsigned int* inc_bits, unsigned int* inc_norm_bits,
+                        const uint32_t* keys,
+                        uint32_t* cell_inc, int C, int nz, UDiv div_z, PlaneArgs pa,
+                        const float4* fdelta, float* pn, ResidualArgs ra) {
+  const int i = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   if (ra.res) {
     // residual mode: x* is left as it is once the sweep found it within the
     // target (the counts that it handed to others are taken back)
@@ -252,9 +255,9 @@ __global__ void __launch_bounds__(256) k_apply(int n, float4* __restrict__ xs, f
 gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStream_t st, const ResidualSlot* res) {
   if (S->n <= 0) return GG_OK;
   prof_begin(S, PC_APPLY, st);
-  // a listed sweep after this one (more) reads the per-cell increments
-  uint32_t* cell_inc = (S->g.cell_inc && more) ? S->g.cell_inc : nullptr;
-  if (cell_inc) GG_CUDA(cudaMemsetAsync(cell_inc, 0, sizeof(uint32_t) * ((size_t)S->grid.C + 1), st));
+  // a listed sweep after this one (more) reads the per-cell increments (the
+  // sweep before cleared the table)
+  uint32_t* cell_inc = (sweep_lists(S) && more) ? S->g.cell_inc[it & 1] : nullptr;
   PlaneArgs pa;
   pa.n = std::max(0, std::min(S->P.n_planes, 8));
   pa.coulomb = S->P.contact_law == 1;
@@ -267,13 +270,11 @@ gg_status apply(gg_system* S, int it, bool stab, bool last, bool more, cudaStrea
   pa.scene_inv_w = S->scene_width > 0.0f ? 1.0f / S->scene_width : 0.0f;
   pa.scene_mu = S->scene_mu;
   const int ta = S->tune.apply_threads;
-  k_apply<<<blocks_for(S->n, ta), ta, 0, st>>>((int)S->n, S->g.xs, S->g.pos[S->g.cur], S->g.delta,
-                                                 S->g.s_extra, S->g.ncon, S->g.contacts, stab ? 1 : 0,
-                                                 last ? 1 : 0, &S->scal->inc_bits[it], &S->scal->inc_norm_bits[it],
-                                                 S->g.keys, cell_inc,
-                                                 S->grid.C, S->grid.nz, make_udiv((uint32_t)S->grid.nz), pa,
-                                                 pa.coulomb ? S->g.fdelta : nullptr, S->g.pn,
-                                                 ResidualArgs{res, &S->scal->res_done, S->P.target_residual, it});
+  GG_CUDA(launch_chained(k_apply, blocks_for(S->n, ta), ta, st, (int)S->n, S->g.xs, S->g.pos[S->g.cur], S->g.delta,
+                         S->g.s_extra, S->g.ncon, S->g.contacts, stab ? 1 : 0, last ? 1 : 0, &S->scal->inc_bits[it],
+                         &S->scal->inc_norm_bits[it], S->g.keys, cell_inc, S->grid.C, S->grid.nz,
+                         make_udiv((uint32_t)S->grid.nz), pa, pa.coulomb ? S->g.fdelta : nullptr, S->g.pn,
+                         ResidualArgs{res, &S->scal->res_done, S->P.target_residual, it}));
   count_launches(S, 1);
   prof_end(S, PC_APPLY, S->n, st);
   GG_CUDA(cudaGetLastError());
@@ -289,9 +290,9 @@ struct FinalArgs {
 // final_velocity_functor (Solver.cu:193-248), final_update (:249-270) and
 // the adaptive_last_step reset (:103-108).
 template <int MM>
-__global__ void k_finalize(int n, float4* __restrict__ pos, const float4* __restrict__ xs,
-                           float4* __restrict__ vel, int32_t* __restrict__ als, FinalArgs f) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_finalize(int n, float4* pos, const float4* xs,
+                           float4* vel, int32_t* als, FinalArgs f) {
+  const int i = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   if (i >= n) return;
   const float4 p = pos[i];
   const float4 x = xs[i];
@@ -327,7 +328,8 @@ gg_status finalize(gg_system* S, cudaStream_t st) {
   prof_begin(S, PC_FINALIZE, st);
   auto kern = S->P.math_mode ? k_finalize<1> : k_finalize<0>;
   const int tf = S->tune.finalize_threads;
-  kern<<<blocks_for(S->n, tf), tf, 0, st>>>((int)S->n, S->g.pos[c], S->g.xs, S->g.vel[c], S->g.als[c], f);
+  GG_CUDA(launch_chained(kern, blocks_for(S->n, tf), tf, st, (int)S->n, S->g.pos[c], S->g.xs, S->g.vel[c],
+                         S->g.als[c], f));
   count_launches(S, 1);
   prof_end(S, PC_FINALIZE, S->n, st);
   GG_CUDA(cudaGetLastError());

@@ -124,8 +124,6 @@ gg_status step_once(gg_system* S) {
   if ((rc = predict(S, st)) != GG_OK) return rc;
   if (S->P.warm_start == 1 && (rc = warm_start_apply(S, st)) != GG_OK) return rc;
   if (S->P.warm_start == 2 && (rc = warm_start_record(S, st)) != GG_OK) return rc;
-  // Coulomb law: the normal correction each particle receives accumulates over the substep
-  if (S->P.contact_law == 1 && S->n > 0) GG_CUDA(cudaMemsetAsync(S->g.pn, 0, sizeof(float) * (size_t)S->n, st));
   if (S->P.target_residual > 0.0f) {
     // residual mode: the stabilisation sweeps, then Jacobi sweeps until the
     // largest penetration, measured before each sweep, is within the target
@@ -218,7 +216,7 @@ static void free_all(gg_system* S) {
   }
   void* ptrs[] = {G.merge_vel, G.surface, G.sdist, G.cover, G.xs, G.inv_m, G.delta, G.s_extra, G.contacts,
                   G.ncon, G.keys, G.perm, G.cell_start, G.cell_surf, G.prop, G.ldens, G.winner, G.split_flag, G.keep_flag,
-                  G.split_slot, G.keep_slot, G.child_pos, G.nl_idx, G.nl_meta, G.nl_acc, G.nl_queue, G.cell_inc, G.ld_sum, G.ld_cnt, G.claim_tgt, G.claimed, G.cell_claim, G.child_cell, G.fdelta, G.pn, S->b.pos, S->b.animated, S->b.pos_alt,
+                  G.split_slot, G.keep_slot, G.child_pos, G.nl_idx, G.nl_meta, G.nl_acc, G.nl_queue, G.cell_inc[0], G.cell_inc[1], G.ld_sum, G.ld_cnt, G.claim_tgt, G.claimed, G.cell_claim, G.child_cell, G.fdelta, G.pn, S->b.pos, S->b.animated, S->b.pos_alt,
                   S->b.animated_alt, S->b.keys, S->b.perm, S->b.cell_start, S->u.keys, S->u.perm, S->scal,
                   S->stats_partial, S->stage, S->feat, S->xs0, S->warm_target, S->scene_fcap,
                   S->scene_acc, S->scene_mu, S->window};
@@ -343,7 +341,8 @@ gg_status system_create(const gg_desc* d, gg_system** out) {
     ALLOC(G.nl_meta, cap);
     ALLOC(G.nl_acc, cap);
     ALLOC(G.nl_queue, cap);
-    ALLOC(G.cell_inc, C1);
+    ALLOC(G.cell_inc[0], C1);
+    ALLOC(G.cell_inc[1], C1);
   }
   ALLOC(S->b.pos, S->nb); ALLOC(S->b.animated, S->nb); ALLOC(S->b.pos_alt, S->nb);
   ALLOC(S->b.animated_alt, S->nb); ALLOC(S->b.keys, S->nb); ALLOC(S->b.perm, S->nb);
