@@ -56,7 +56,7 @@ struct DevScalars {
   unsigned int disp0_bits;     // max |dt v| of the predict (float bits)
   unsigned int tile_fallback;  // sweep blocks that could not use the shared-memory tile
   int nl_queued[kMaxSweeps];          // per sweep: particles whose contact list is rebuilt
-  int nl_over[kMaxSweeps];     // per sweep: particles with more candidates than a list holds
+  int nl_over;                 // long contact lists handed out in this substep
   ResidualSlot res[kMaxSweeps];  // residual mode, per sweep
   int res_done;                // residual mode: 1 + the sweep whose x* met the target (later sweeps do nothing)
   unsigned int pen_bits;       // residual mode: largest penetration (float bits)
@@ -70,7 +70,7 @@ struct DevScalars {
   int n_split;
   int n_split_appended;
   int n_kept;
-  unsigned long long nlist_rebuilds;  // listed-sweep list builds (not reset per substep)
+  unsigned long long nlist_rebuilds;  // listed-sweep list builds, counted while profiling (not reset per substep)
 };
 
 
@@ -80,6 +80,7 @@ constexpr int kMergeMaxIter = 64;  // claim-status iterations of the merge sched
 // Largest element count of a set: launches round counts up to whole tiles
 // of at most 4,096 items and index them with signed 32-bit integers.
 constexpr int64_t kMaxCount = ((int64_t)1 << 31) - ((int64_t)1 << 16);
+constexpr int64_t kLongInts = 4;
 constexpr int kNlistMax = 64;  // contact candidates kept per particle (walls within reach included)
 
 // Kernel classes timed by gg_profile_*.
@@ -107,7 +108,6 @@ struct Granular {
   // recomputed every step
   int32_t* surface = nullptr;
   float* sdist = nullptr;
-  float4* cover = nullptr;
   float4* xs = nullptr;       // predicted positions x*, w = contact radius
   float* inv_m = nullptr;     // 1 / (m exp(-y))
   float4* delta = nullptr;    // sweep output: dx, dy, dz, packed counts
@@ -117,6 +117,7 @@ struct Granular {
   int32_t* nl_idx = nullptr;  // contact candidate lists [kNlistMax][cap]
   int4* nl_meta = nullptr;    // query cell at list build, entry count (-1 = overflow)
   float* nl_acc = nullptr;    // displacement bound summed since the particle's list build
+  int32_t* nl_long = nullptr;  // long contact lists: kLongInts a particle in all, shared out to those that need one
   int32_t* nl_queue = nullptr; // particles whose list is rebuilt in this sweep
   // per cell (C+1): max |x* increment| of its particles in a sweep (float
   // bits); the sweeps take turns, the next one reading the last one's

@@ -64,11 +64,14 @@ struct SweepArgsT<true> {
   int4* __restrict__ nl_meta;
   float* __restrict__ nl_acc;
   int32_t* __restrict__ nl_queue;
-  int32_t* __restrict__ nl_over;  // particles with more candidates than a list holds, left to the groups
+  int32_t* __restrict__ nl_over;  // particles with long lists, left to the groups
+  int32_t* __restrict__ nl_long;  // the long lists, kLongMax entries each
+  int long_rows;
   size_t li_row, li_step;  // entry k of particle i's list: nl_idx[i * li_row + k * li_step]
   const uint32_t* __restrict__ cell_inc;  // the last sweep's increments
   uint32_t* __restrict__ cell_clear;  // the table of this sweep's, to be cleared (two take turns)
   ResidualSlot* __restrict__ res;  // residual mode: this sweep's penetrations (kernels with bit 2 of MM)
+  int count_builds;  // profiling: count the lists built
   int group_queue;  // queues up to this length are rebuilt by groups
   float skin;
   float eabs;  // bound on the rounding of one position update
@@ -109,10 +112,13 @@ struct SweepArgsT<false> {
   float* nl_acc;
   int32_t* nl_queue;
   int32_t* nl_over;
+  int32_t* nl_long;
+  int long_rows;
   size_t li_row, li_step;
   const uint32_t* cell_inc;
   uint32_t* cell_clear;
   ResidualSlot* res;
+  int count_builds;
   int group_queue;
   float skin;
   float eabs;
@@ -568,9 +574,12 @@ __global__ void __launch_bounds__(kWarpThreads) k_sweep_list(SweepArgsRO a) {
 // apply kernel) over the 27 stencil cells and the particle's own cell.
 // Lists whose bound runs out are rebuilt; the others are kept.
 
-// nl_meta[i].w: the list's length, with a flag when it holds walls; -1 when
-// there were too many candidates to list.
-constexpr int kNlistWalls = 1 << 16, kNlistCount = kNlistWalls - 1;
+// nl_meta[i].w: the list's length, with flags when it holds walls and when it
+// is a long one; or why there is none.  From kNlistLong up it is the groups'.
+constexpr int kNlistWalls = 1 << 16, kNlistLong = 1 << 17, kNlistCount = kNlistWalls - 1;
+constexpr int kNlistNone = 1 << 18;  // too many for a long one (or all are taken): the groups scan every sweep
+constexpr int kNlistNew = -1;        // too many candidates for a list of kNlistMax: the groups make a long one
+constexpr int kNlistAgain = -2;      // the same, found in a short queue: queued again at the next sweep
 
 // The listed candidates in order, with the next entry's gathers issued
 // before the current one is processed.  entry(k) gives the k-th entry: a
@@ -665,9 +674,10 @@ __device__ __forceinline__ float nlist_cell_bound(const Args& a, int3 q, uint32_
 // Sweeps after the first: particles whose list is still exact run it; the
 // others are queued for k_sweep_nlist_build.
 // 5 resident blocks of 256 (48 registers; the per-target state carries no
-// double, and a few bytes spill): about 2 % faster than 4 blocks at 64.
+// double, and a few bytes spill): about 2 % faster than 4 blocks at 64 in the
+// large systems that are launched plainly.
 template <int MM, class Args>
-__global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(Args a) {
+__global__ void __launch_bounds__(256, std::is_same<Args, SweepArgs>::value ? 4 : 5) k_sweep_nlist_keep(Args a) {
   const Grid& g = a.g;
   const int tid = sweep_thread<Args>();
   if ((MM & 4) && a.scal->res_done) return;
@@ -680,12 +690,14 @@ __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(Args a) {
     const int3 q = trunc_cell(g, f3(xi4));
     const int4 m = a.nl_meta[i];
     bool keep = false;
-    if (m.w >= 0 && m.x == q.x && m.y == q.y && m.z == q.z) {
+    rebuild = m.w < kNlistLong;
+    if ((unsigned)m.w < (unsigned)kNlistLong && m.x == q.x && m.y == q.y && m.z == q.z) {
       const float A0 = a.nl_acc[i];
       float A = A0 + nlist_step(a, __uint_as_float(a.scal->inc_norm_bits[a.it - 1]));
       if (!nlist_bound_ok(a, A)) A = A0 + nlist_step(a, nlist_cell_bound(a, q, a.keys[i]));
       if (nlist_bound_ok(a, A)) {
         keep = true;
+        rebuild = false;
         a.nl_acc[i] = A;
       }
     }
@@ -697,8 +709,6 @@ __global__ void __launch_bounds__(256, 5) k_sweep_nlist_keep(Args a) {
       const int32_t* li = a.nl_idx + i;
       apply_entries<MM>(a, t, m.w & kNlistCount, [&](int k) { return __ldcs(li + k * a.li_step); }, u, pen);
       store_sums<MM>(a, i, u);
-    } else {
-      rebuild = true;
     }
   }
   // The block's rebuilds go to the queue together, in index order: the
@@ -811,8 +821,9 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(Args a, 
       }
     });
     if (cnt > kNlistMax) {
-      // too many candidates to list: the groups run them
-      a.nl_over[atomicAdd(&a.scal->nl_over[a.it], 1)] = i;
+      // too many candidates to list here: the groups take over
+      a.nl_meta[i] = make_int4(0, 0, 0, kNlistNew);
+      a.nl_over[atomicAdd(&a.scal->nl_over, 1)] = i;
       continue;
     }
     a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, cnt | (walls ? kNlistWalls : 0));
@@ -837,57 +848,86 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(Args a, 
 // reference's order, one lane to a component.  A list that runs out is
 // rebuilt by its own group in the same launch.  Lists are then stored
 // particle by particle.  A particle with more candidates than a list holds
-// runs each full list as the scan goes on, and scans again at the next
-// sweep.
-constexpr int kGroupThreads = 256;
-
+// runs each full list as the scan goes on, and gets a long list, of kLongMax
+// entries, as long as there are any.
 //
-// kQueue: rebuilds the particles of a queue instead: the whole one if it is
-// short, else (the threads have built those lists) the particles whose
-// candidates a list does not hold.
-template <int MM, int G, bool kQueue>
-__global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
-  constexpr unsigned kAll = 0xffffffffu;
-  constexpr int kGroups = kGroupThreads / G;
-  constexpr int NC = (MM & 2) ? 6 : 3;  // components of a share
+// Measured on a GB300 against one thread to a particle (same bits): a frame
+// of 4 substeps of 1,000 particles 1.90 to 0.92 ms, of 32,768 particles 2.2
+// to 0.91 ms; a substep of the box scene (51,000 particles, 2.5 M render
+// points) 2.19 to 1.66 ms.  With the queues of the thread kernels: two
+// substeps of 16 settled scenes (643,000 particles) 9.6 to 5.6 ms, a queued
+// rebuild launch 800 to about 60 us there.  8 lanes are bound by issue (the
+// target's values are computed by every lane of a group), 32 by latency.
+//
+// The work is all particles, or (k_sweep_rest) what the thread kernels leave:
+// the particles with long lists, nl_over, in the order of their lists, checked
+// and run in the same way, and the rebuilds of a short queue.
+constexpr int kGroupThreads = 256;
+constexpr int kLongMax = 160;
+
+enum GroupWork { kWorkAll, kWorkLong, kWorkQueue };
+
+// The shared memory of a block's groups (a kernel's kinds of work take turns
+// in it).
+template <int MM, int G>
+struct GroupSmem {
+  static constexpr int kGroups = kGroupThreads / G;
+  static constexpr int kStep = 2 * G;              // candidates of a scan step, two a lane
+  static constexpr int NC = (MM & 2) ? 6 : 3;      // components of a share
   // a group's rows of shares, padded so that the groups of a warp use
   // different banks
-  constexpr int kRow = G == 8 ? (NC == 6 ? 56 : 24) : G == 16 ? (NC == 6 ? 112 : 48) : NC * G;
-  constexpr int kStep = 2 * G;  // candidates of a scan step
-  __shared__ int32_t s_list[kGroups][kNlistMax + kStep];
-  __shared__ int4 s_col[kGroups][9];
-  __shared__ float s_share[kGroups][kRow];
+  static constexpr int kRow = G == 8 ? (NC == 6 ? 56 : 24) : G == 16 ? (NC == 6 ? 112 : 48) : NC * G;
+  int4 col[kGroups][9];
+  int32_t list[kGroups][kNlistMax + kStep];
+  float share[kGroups][kRow];
+};
+
+template <int MM, int G, GroupWork kWork>
+__device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* smem, Penetration& pen) {
+  using Smem = GroupSmem<MM, G>;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kGroups = Smem::kGroups, NC = Smem::NC, kStep = Smem::kStep, kAhead = kStep / G;
+  auto& s_list = static_cast<Smem*>(smem)->list;
+  auto& s_col = static_cast<Smem*>(smem)->col;
+  auto& s_share = static_cast<Smem*>(smem)->share;
   const Grid& g = a.g;
-  const int tid = (int)pdl_wait(threadIdx.x), lane = tid & 31, gl = lane & (G - 1), grp = tid / G;
+  const int lane = tid & 31, gl = lane & (G - 1), grp = tid / G;
   const unsigned glt = (1u << gl) - 1u;
   auto gballot = [&](bool p) {
     const unsigned b = __ballot_sync(kAll, p);
     return G == 32 ? b : (b >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u);
   };
-  if ((MM & 4) && a.scal->res_done) return;
-  if (!kQueue) clear_increments(a, tid);
-  Penetration pen;
   int total = a.n;
-  const int32_t* queue = nullptr;
-  if (kQueue) {
-    const int queued = a.it > 0 ? a.scal->nl_queued[a.it] : INT_MAX;
-    queue = queued <= a.group_queue ? a.nl_queue : a.nl_over;
-    total = queued <= a.group_queue ? queued : a.scal->nl_over[a.it];
+  if (kWork == kWorkLong) total = a.scal->nl_over;
+  if (kWork == kWorkQueue) {
+    total = a.scal->nl_queued[a.it];
+    if (total > a.group_queue) return;  // the threads took it
   }
-  for (int base = blockIdx.x * kGroups; base < total; base += gridDim.x * kGroups) {
-  const int slot = base + grp;
-  const bool act = slot < total;
+  // a warp's groups at a time, the warps of a block on their own (the work of
+  // one differs much from that of the next)
+  constexpr int kWarpGroups = 32 / G;
+  for (int base = (blockIdx.x * (kGroupThreads / 32) + (tid >> 5)) * kWarpGroups; base < total;
+       base = kWork == kWorkAll ? total : base + (int)gridDim.x * kGroups) {
+  const int own = base + (lane / G);
+  const bool act = own < total;
   // (groups past the end follow along and write nothing)
-  const int is = kQueue ? queue[act ? slot : total - 1] : (act ? slot : total - 1), i = act ? is : -1;
+  const int slot = act ? own : total - 1;
+  const int is = kWork == kWorkAll ? slot : kWork == kWorkLong ? a.nl_over[slot] : a.nl_queue[slot];
+  const int i = act ? is : -1;
   Target t;
   make_target_lite(a, is, a.xs[is], t);
   int cnt = 0;
-  bool walls = false, rebuild = act;
-  if (!kQueue && a.it > 0) {
+  bool walls = false, rebuild = act, counted = true;
+  // the long list, and where this one is: -1 none yet, -2 none to be had
+  int long_row = kWork == kWorkAll ? -1 : kWork == kWorkLong && slot < a.long_rows ? slot : -2;
+  int32_t* row = a.nl_idx + is * a.li_row;
+  if (kWork == kWorkLong || (kWork == kWorkAll && a.it > 0)) {
     const int4 m = a.nl_meta[is];
-    const bool same = act && m.w >= 0 && m.x == t.q.x && m.y == t.q.y && m.z == t.q.z;
+    if (kWork == kWorkAll && m.w >= 0 && (m.w & kNlistLong)) long_row = row[0];
+    counted = m.w != kNlistNew;  // (the threads that left it counted it)
+    const bool same = act && m.w >= 0 && m.w != kNlistNone && m.x == t.q.x && m.y == t.q.y && m.z == t.q.z;
     const float A0 = a.nl_acc[is];
-    float A = A0 + nlist_step(a, __uint_as_float(a.scal->inc_norm_bits[a.it - 1]));
+    float A = A0 + nlist_step(a, __uint_as_float(a.scal->inc_norm_bits[max(a.it, 1) - 1]));
     bool ok = same && nlist_bound_ok(a, A);
     const bool need = same && !ok;
     if (__any_sync(kAll, need)) {
@@ -901,6 +941,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
       rebuild = false;
       cnt = m.w & kNlistCount;
       walls = (m.w & kNlistWalls) != 0;
+      if (m.w & kNlistLong) row = a.nl_long + (size_t)long_row * kLongMax;
       if (gl == 0) a.nl_acc[i] = A;
     }
   }
@@ -921,8 +962,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
   __syncwarp();
   const float Bs = t.Bf + a.skin, Bs2 = Bs * Bs * 1.0001f;
   const float rcs = t.rc + a.skin;
-  int32_t* row = a.nl_idx + is * a.li_row;
   bool over = false;
+  int stored = 0;  // entries in the long list
   float sum = 0.0f;  // component gl of the corrections
   int c = 0, s_loc = 0;
   // the scan's place (the same for all groups of a warp): column and cell,
@@ -942,9 +983,29 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
         nb = in ? a.bcs[col.z + z + 1] - b0 : 0;
       }
       bool full = false;
-      for (; __any_sync(kAll, v - gl < nb + np); v += kStep) {
-        if ((full = __any_sync(kAll, cnt > kNlistMax && rebuild))) break;
+      if (G < 32 && !__any_sync(kAll, nb > 0)) {
+        // particles alone: a step's loads in flight together (small groups
+        // take many steps; to a whole warp the shorter code is worth more)
+        for (; __any_sync(kAll, v - gl < np); v += kStep) {
+          if ((full = __any_sync(kAll, cnt > kNlistMax && rebuild))) break;
+          float4 xj[kAhead];
 #pragma unroll
+          for (int u = 0; u < kAhead; ++u) xj[u] = a.xs[v + u * G < np ? j0 + v + u * G : is];
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) {
+            const float dx = t.x.x - xj[u].x, dy = t.x.y - xj[u].y, dz = t.x.z - xj[u].z;
+            const float rs = rcs + xj[u].w;
+            const int e = j0 + v + u * G;
+            const bool hit = v + u * G < np && e != i &&
+                             !(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz))) > rs * rs * 1.0001f);
+            const unsigned hb = gballot(hit);
+            if (hit) s_list[grp][cnt + __popc(hb & glt)] = e;
+            cnt += __popc(hb);
+          }
+        }
+      } else for (; __any_sync(kAll, v - gl < nb + np); v += kStep) {
+        if ((full = __any_sync(kAll, cnt > kNlistMax && rebuild))) break;
+#pragma unroll 1
         for (int u = 0; u < kStep; u += G) {
           const int w = v + u;
           bool hit = false;
@@ -979,11 +1040,32 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
     const bool filled = rebuild && cnt > kNlistMax;
     over |= filled;
     __syncwarp();
-    if (done && rebuild) {
-      if (!over)
+    if (kWork == kWorkAll && __any_sync(kAll, filled && long_row == -1)) {
+      int r = 0;
+      if (filled && long_row == -1 && gl == 0) r = atomicAdd(&a.scal->nl_over, 1);
+      r = __shfl_sync(kAll, r, 0, G);
+      if (filled && long_row == -1) long_row = r < a.long_rows ? r : -2;
+    }
+    if (rebuild && (filled || done)) {
+      // (a particle that has a long list keeps to it)
+      if (over || long_row >= 0) {
+        if (stored + cnt > kLongMax) long_row = -2;
+        if (long_row >= 0)
+          for (int k = gl; k < cnt; k += G) a.nl_long[(size_t)long_row * kLongMax + stored + k] = s_list[grp][k];
+        stored += cnt;
+      } else {
         for (int k = gl; k < cnt; k += G) row[k * a.li_step] = s_list[grp][k];
-      if (gl == 0) {
-        a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, over ? -1 : cnt | (walls ? kNlistWalls : 0));
+      }
+      if (done && gl == 0) {
+        int w = cnt;
+        if (long_row >= 0) {
+          w = stored | kNlistLong;
+          if (kWork == kWorkAll) row[0] = long_row;
+        } else if (over || kWork == kWorkLong) {
+          w = kWork == kWorkQueue ? kNlistAgain : kNlistNone;
+        }
+        if (walls && w >= 0 && w != kNlistNone) w |= kNlistWalls;
+        a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, w);
         a.nl_acc[i] = 0.0f;
       }
     }
@@ -1034,9 +1116,45 @@ __global__ void __launch_bounds__(kGroupThreads) k_sweep_group(SweepArgs a) {
       if (gl == 6) out[3] = __int_as_float(c);
     }
   }
-  const int built = __syncthreads_count(rebuild && gl == 0);
-  if (threadIdx.x == 0 && built && queue != a.nl_over)  // (those are counted by the threads that left them)
-    atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)built);
+  if (a.count_builds) {
+    const unsigned b = __ballot_sync(kAll, rebuild && counted && gl == 0);
+    if (lane == 0 && b) atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)__popc(b));
+  }
+  __syncwarp();
+  }
+}
+
+template <int MM, int G>
+__global__ void __launch_bounds__(kGroupThreads, 3) k_sweep_group(SweepArgs a) {
+  const int tid = (int)pdl_wait(threadIdx.x);
+  if ((MM & 4) && a.scal->res_done) return;
+  clear_increments(a, tid);
+  __shared__ GroupSmem<MM, G> smem;
+  Penetration pen;
+  sweep_groups<MM, G, kWorkAll>(a, tid, &smem, pen);
+  if (MM & 4) store_penetration(a, pen);
+}
+
+// What the thread kernels leave: the long lists, by whole warps (their scans
+// and lists are long), and short queues, by whole warps as well where
+// particles lie so close that one in 256 has a long list, else by groups of
+// 8: 16 settled scenes 4.90 ms with 8 and 4.63 with 32, a settled pile 2.44
+// and 2.28, but a loosely packed warm-started solve 4.6 and 5.6.
+template <int MM>
+__global__ void __launch_bounds__(kGroupThreads, 3) k_sweep_rest(SweepArgs a) {
+  const int tid = (int)pdl_wait(threadIdx.x);
+  if ((MM & 4) && a.scal->res_done) return;
+  __shared__ union {
+    GroupSmem<MM, 32> wide;
+    GroupSmem<MM, 8> narrow;
+  } smem;
+  Penetration pen;
+  sweep_groups<MM, 32, kWorkLong>(a, tid, &smem, pen);
+  if (a.it > 0) {
+    const bool wide = a.scal->nl_over > (a.n >> 8);
+    __syncthreads();  // the warps lay their shared memory out differently
+    if (wide) sweep_groups<MM, 32, kWorkQueue>(a, tid, &smem, pen);
+    else sweep_groups<MM, 8, kWorkQueue>(a, tid, &smem, pen);
   }
   if (MM & 4) store_penetration(a, pen);
 }
@@ -1109,7 +1227,7 @@ constexpr int64_t kGroup32Max = 4096, kGroup16Max = 16384;
 
 template <int G>
 static void launch_group(const SweepArgs& a, int mm, cudaStream_t st) {
-  auto kern = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, G, false>);
+  auto kern = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, G>);
   launch_chained(kern, blocks_for(a.n, kGroupThreads / G), kGroupThreads, st, a);
 }
 
@@ -1160,8 +1278,11 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
   a.cell_inc = S->g.cell_inc[(it & 1) ^ 1];
   a.cell_clear = S->g.cell_inc[it & 1];
   a.nl_over = S->g.split_slot;  // (scratch of the split, free during the sweeps)
+  a.nl_long = S->g.nl_long;
+  a.long_rows = (int)std::min<int64_t>(kLongInts * S->cap / kLongMax, INT_MAX);
   a.li_row = a.li_step = 0;
   a.group_queue = 0;
+  a.count_builds = S->profiling ? 1 : 0;
   a.skin = S->nl_skin;
   a.div_yz = make_udiv((uint32_t)(S->grid.ny * S->grid.nz));
   a.div_z = make_udiv((uint32_t)S->grid.nz);
@@ -1209,7 +1330,7 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
       count_launches(S, 1);
     }
     // short queues, and what a list does not hold
-    auto rest = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, 8, true>);
+    auto rest = GG_SWEEP_KERNEL(mm, k_sweep_rest<MM>);
     launch_chained(rest, S->num_sms * 3, kGroupThreads, st, a);
     count_launches(S, 1);
   } else {

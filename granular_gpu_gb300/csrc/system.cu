@@ -214,7 +214,7 @@ static void free_all(gg_system* S) {
     cudaFree(G.merge_count[k]); cudaFree(G.remove[k]); cudaFree(G.als[k]);
     cudaFree(S->u.pos[k]); cudaFree(S->u.vel[k]);
   }
-  void* ptrs[] = {G.merge_vel, G.surface, G.sdist, G.cover, G.xs, G.inv_m, G.delta, G.s_extra, G.contacts,
+  void* ptrs[] = {G.merge_vel, G.surface, G.sdist, G.nl_long, G.xs, G.inv_m, G.delta, G.s_extra, G.contacts,
                   G.ncon, G.keys, G.perm, G.cell_start, G.cell_surf, G.prop, G.ldens, G.winner, G.split_flag, G.keep_flag,
                   G.split_slot, G.keep_slot, G.child_pos, G.nl_idx, G.nl_meta, G.nl_acc, G.nl_queue, G.cell_inc[0], G.cell_inc[1], G.ld_sum, G.ld_cnt, G.claim_tgt, G.claimed, G.cell_claim, G.child_cell, G.fdelta, G.pn, S->b.pos, S->b.animated, S->b.pos_alt,
                   S->b.animated_alt, S->b.keys, S->b.perm, S->b.cell_start, S->u.keys, S->u.perm, S->scal,
@@ -323,7 +323,7 @@ gg_status system_create(const gg_desc* d, gg_system** out) {
     ALLOC(G.merge_count[k], cap); ALLOC(G.remove[k], cap); ALLOC(G.als[k], cap);
     ALLOC(S->u.pos[k], S->nu); ALLOC(S->u.vel[k], S->nu);
   }
-  ALLOC(G.merge_vel, cap); ALLOC(G.surface, cap); ALLOC(G.sdist, cap); ALLOC(G.cover, cap);
+  ALLOC(G.merge_vel, cap); ALLOC(G.surface, cap); ALLOC(G.sdist, cap);
   ALLOC(G.xs, cap); ALLOC(G.inv_m, cap); ALLOC(G.delta, cap); ALLOC(G.s_extra, cap);
   ALLOC(G.contacts, cap); ALLOC(G.ncon, cap); ALLOC(G.keys, cap); ALLOC(G.perm, cap);
   ALLOC(G.cell_start, C1); ALLOC(G.cell_surf, C1); ALLOC(G.prop, cap); ALLOC(G.ldens, cap); ALLOC(G.winner, cap);
@@ -338,6 +338,7 @@ gg_status system_create(const gg_desc* d, gg_system** out) {
   if (!(S->nl_skin > 0.0f) || !std::isfinite(S->nl_skin)) S->nl_skin = 0.0f;
   if (S->nl_skin > 0.0f) {
     ALLOC(G.nl_idx, (int64_t)kNlistMax * cap);
+    ALLOC(G.nl_long, kLongInts * cap);
     ALLOC(G.nl_meta, cap);
     ALLOC(G.nl_acc, cap);
     ALLOC(G.nl_queue, cap);

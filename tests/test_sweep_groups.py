@@ -61,3 +61,35 @@ def test_overlong_lists_match_oracle(n, spacing, law):
 def test_thread_kernels_and_their_queues_match_oracle(n, spacing, law):
     most = _check(_scene(n, spacing, law), 2)
     assert most > 64 or spacing > 0.8
+
+
+@pytest.mark.parametrize("law", [0, 1])
+@pytest.mark.parametrize("n", [600, 9000, 30000, 101000])
+@pytest.mark.parametrize("spacing", [1.3, 1.15, 0.95, 0.8])
+def test_long_lists_match_oracle(n, spacing, law):
+    """A skin of 1.2 r and spacings that list from about 60 to about 250
+    candidates: lists of both kinds kept over the sweeps, long ones that stay
+    long, and more than a long one holds."""
+    d = _scene(n, spacing, law)
+    d["params"].nlist_skin = 0.012
+    d["params"].stab_iters, d["params"].iters = 1, 5
+    _check(d, 1)
+
+
+def test_long_lists_are_kept_and_run_out():
+    """Fewer long lists than particles that want one: with room for two
+    long lists (a capacity of 100 particles) the others scan every sweep."""
+    d = _scene(100, 1.0, 0)
+    d["params"].nlist_skin = 0.014
+    d["params"].iters = 6
+    d["max_particles"] = 100
+    _check(d, 2)
+    d = _scene(20000, 1.15, 0)
+    d["params"].nlist_skin, d["params"].iters = 0.014, 6
+    d["gravity"] = (0.0, 0.0, 0.0)
+    s = gg.GranularSystem(**workloads.system_kwargs(d), device=0)
+    s.profile_begin()
+    s.step(1)
+    built = s.profile_end()["_nlist_rebuilds"]
+    assert built < 7 * 20000, "every sweep rebuilt every list"
+    s.close()
