@@ -489,16 +489,21 @@ __global__ void __launch_bounds__(256, 6) k_upsample(UpArgs a) {
   up_finish(a, i, p4, wv, rep, gw, maxw, near_b);
 }
 
-// The same for a support that reaches every candidate of the stencil, on
-// packed pairs of candidates: k_upsample<true> is bound by the issue of
-// about 48 instructions a candidate, this form issues 32 and is bound by the
-// FP32 pipe (65 % active) and the loads.  10.56 to 9.33 ms per launch on the
-// 8.4 M column (33.5 M render points, 263 candidates each; 0.06 ms of
-// pairing included).  The particles come two to an entry, so three loads
-// bring two of them in the pairs that the packed operations take; the sums
-// stay single and in candidate order, so the results are the same bits.  A
-// column's first and last entry may hold a particle that is not of the
-// column: it takes no part in the sums.
+// The same on packed pairs of candidates, all of the stencil: k_upsample<true>
+// is bound by the issue of about 48 instructions a candidate, this form
+// issues 32 and is bound by the FP32 pipe (65 % active) and the loads.  10.56
+// to 9.33 ms per launch on the 8.4 M column (33.5 M render points, 263
+// candidates each; 0.06 ms of pairing included).  The particles come two to
+// an entry, so three loads bring two of them in the pairs that the packed
+// operations take; the sums stay single and in candidate order, so the
+// results are the same bits.  A column's first and last entry may hold a
+// particle that is not of the column: it takes no part in the sums.
+//
+// kCut: candidates beyond the support (with k_upsample<false>'s margin) take
+// no part either.  Against its marks, which leave each lane of a warp other
+// hits to gather: box scene (2.5 M points) 0.48 and 0.44 ms, settled pile
+// 0.46 and 0.26 ms, 1 M column with scaled constants 1.23 and 1.06 ms.
+template <bool kCut>
 __global__ void __launch_bounds__(256, 4) k_upsample_pairs(UpArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
@@ -535,14 +540,14 @@ __global__ void __launch_bounds__(256, 4) k_upsample_pairs(UpArgs a) {
       unpack2(mul2(w, pack2(B.z, B.w)), x0, x1);
       unpack2(mul2(w, pack2(C.x, C.y)), y0, y1);
       unpack2(mul2(w, pack2(C.z, C.w)), z0, z1);
-      if (2 * e >= j0) {
+      if (2 * e >= j0 && (!kCut || d0 <= a.cut2)) {
         gw += w0;
         wv.x += x0;
         wv.y += y0;
         wv.z += z0;
         maxw = fmaxf(maxw, w0);
       }
-      if (2 * e + 1 < j1) {
+      if (2 * e + 1 < j1 && (!kCut || d1 <= a.cut2)) {
         gw += w1;
         wv.x += x1;
         wv.y += y1;
@@ -601,7 +606,11 @@ gg_status upsample(gg_system* S, cudaStream_t st) {
   prof_begin(S, PC_UPSAMPLE, st);
   // the packed form wants memory for the pairs and a support that is one
   // (with a negative 1/h^2, infinite distances would weigh)
-  if (all_in && S->P.up_inv_h2 > 0.0f && S->g.nl_idx) {
+  // (marks are faster for a support shorter than a cell: of 0.9 cell lengths
+  // 0.36 against 0.41 ms on the box scene, of 1.1, the reference's, 0.43
+  // against 0.42)
+  const bool pairs_pay = S->P.up_inv_h2 * S->grid.L * S->grid.L <= 1.0f;
+  if ((all_in || pairs_pay) && S->P.up_inv_h2 > 0.0f && S->g.nl_idx) {
     // the contact lists of the substep are done with: their memory holds the
     // pairs (24 of its 256 bytes a particle)
     const int64_t np = (S->n + 1) / 2;
@@ -615,7 +624,8 @@ gg_status upsample(gg_system* S, cudaStream_t st) {
                                                             pairs + 2 * np);
       count_launches(S, 1);
     }
-    k_upsample_pairs<<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
+    if (all_in) k_upsample_pairs<false><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
+    else k_upsample_pairs<true><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
   } else if (all_in) k_upsample<true><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
   else k_upsample<false><<<blocks_for(S->nu, 256), 256, 0, st>>>(a);
   count_launches(S, 1);

@@ -26,12 +26,17 @@ def test_packed_square_root_equals_sqrtf_for_every_float(tmp_path):
 
 @pytest.mark.parametrize("counts", [(1, 1, 1), (2, 1, 1), (3, 1, 1), (5, 7, 9), (12, 11, 13)])
 @pytest.mark.parametrize("odd", ["", "coincident", "nan", "far"])
-def test_whole_stencil_render_points_match_oracle(counts, odd):
-    """The support covers the stencil (0.045 at cells of 0.00808); odd and
-    even particle counts and columns; a render point on a particle, a NaN
-    particle, a particle far from the cell it was binned in."""
-    d = workloads.column_collapse(counts, adaptive=0, upsample_per=4, constants="reference", skip=True)
+@pytest.mark.parametrize("constants", ["reference", "scaled"])
+def test_render_points_match_oracle(counts, odd, constants):
+    """The support covers the stencil (0.045 at cells of 0.00808) or 1.1
+    cells; odd and even particle counts and columns; a render point on a
+    particle, a NaN particle, a particle far from the cell it was binned in."""
+    d = workloads.column_collapse(counts, adaptive=0, upsample_per=4, constants=constants, skip=True)
     d["params"].math_mode = 1
+    if odd == "nan" and constants == "scaled":
+        # the oracle weighs a NaN particle with 0 and adds 0 x NaN; the library
+        # leaves out candidates that are not within the support, NaN ones too
+        pytest.skip("beyond a support shorter than the stencil the library and the oracle treat NaN differently")
     p, u = d["particles"], d["upsampled"]
     if odd == "coincident":
         u[: len(p)] = p
@@ -50,5 +55,24 @@ def test_whole_stencil_render_points_match_oracle(counts, odd):
             a, b = s.read(f, gg.SET_UPSAMPLED), o.read(f, abi.SET_UPSAMPLED)
             assert np.array_equal(a, b, equal_nan=True), f"step {k}, field {f}"
         assert np.array_equal(s.read(gg.FIELD_POS), o.read(abi.FIELD_POS), equal_nan=True)
+    s.close()
+    o.close()
+
+
+@pytest.mark.parametrize("reach", [0.4, 0.95, 0.9999, 1.0001, 1.3, 1.9, 3.5])
+@pytest.mark.parametrize("skin", [-1.0, 0.0])
+def test_supports_of_all_lengths_match_oracle(reach, skin):
+    """Supports of `reach` cells: marks and pairs on both sides of the line,
+    and systems without contact lists, which have no pairs."""
+    d = workloads.column_collapse((9, 10, 11), adaptive=0, upsample_per=3, constants="scaled", skip=True)
+    d["params"].math_mode, d["params"].nlist_skin = 1, skin
+    d["params"].up_inv_h2 = 1.0 / (reach * float(d["cell_length"])) ** 2
+    s = gg.GranularSystem(**workloads.system_kwargs(d), device=0)
+    o = orc.OracleSystem(d, fp64=False)
+    for k in range(2):
+        s.step(1)
+        o.step(1)
+        for f in (gg.FIELD_POS, gg.FIELD_VEL):
+            assert np.array_equal(s.read(f, gg.SET_UPSAMPLED), o.read(f, abi.SET_UPSAMPLED)), f"step {k}, field {f}"
     s.close()
     o.close()
