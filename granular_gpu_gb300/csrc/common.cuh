@@ -144,6 +144,20 @@ __device__ __forceinline__ unsigned int fbits_abs_max(float a, float b) {
   return __float_as_uint(fmaxf(fabsf(a), fabsf(b)));
 }
 
+// Masks of the candidates of a chunk that are within reach, built from the
+// signs of t = reach^2 - distance^2: one funnel shift a candidate, where a
+// comparison takes three instructions to reach its bit.  A NaN (positive as
+// CUDA's operations produce it) counts as within.  near_mask: candidate b of
+// cn (1 to 32) in bit b.
+__device__ __forceinline__ unsigned push_far(unsigned far, float t) {
+  return __funnelshift_l(__float_as_uint(t), far, 1);
+}
+__device__ __forceinline__ unsigned near_mask(unsigned far, int cn) { return __brev(~far) >> (32 - cn); }
+// t, with d's square taken from the reach's
+__device__ __forceinline__ float reach_left(float reach2, float3 d) {
+  return __fmaf_rn(-d.x, d.x, __fmaf_rn(-d.y, d.y, __fmaf_rn(-d.z, d.z, reach2)));
+}
+
 // Warp-aggregated atomicMax of a non-negative float stored as bits.  NaN
 // bits compare above every finite value, so a NaN disables pruning.  The
 // value only grows, so a warp whose maximum does not exceed a value already

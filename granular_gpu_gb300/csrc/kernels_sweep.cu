@@ -22,8 +22,9 @@
 // of a substep: a group of lanes to a particle in small systems
 // (k_sweep_group), a thread to a particle in large ones
 // (k_sweep_nlist_build / k_sweep_nlist_keep, with short rebuild queues and
-// overlong lists left to groups); without lists, k_sweep_list scans the 27 cells; k_sweep is the pruned one-thread-per-
-// particle scan the autotuner may pick where lists do not pay.
+// overlong lists left to groups, k_sweep_rest); without lists, k_sweep_list
+// scans the 27 cells; k_sweep is the pruned one-thread-per-particle scan the
+// autotuner may pick where lists do not pay.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -771,32 +772,28 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(Args a, 
       if (cnt < kNlistMax) li[cnt * a.li_step] = e;
       ++cnt;
     };
-    // candidates in chunks of 32: a mask of those within the reach of the
-    // largest contact radius of the substep, then, in index order, the
-    // exact reach test for each and the pushes
-    const float rmax = __uint_as_float(a.scal->rmax_bits);
-    const float wide = (rcs + rmax) * (rcs + rmax) * 1.0001f;
+    // candidates in chunks of 32: a mask of those within their own reach
+    // (1.00005 squared covers the roundings), then the pushes in index order.
+    // Against a mask for the largest radius by comparisons and an exact test
+    // of each hit, sweeps per substep: 8.4 M particles 9.65 to 9.18 ms,
+    // 655,000 4.13 to 3.74 (unrolled by 8 9.27 and 3.77)
+    const float rcm = rcs * 1.00005f;
     auto scan_particles = [&](int j0, int j1) {
       for (int c0 = j0; c0 < j1; c0 += 32) {
         const int cn = min(32, j1 - c0);
-        unsigned mask = 0u;
+        unsigned far = 0u;
 #pragma unroll 4
         for (int b = 0; b < cn; ++b) {
           const float4 xj = a.xs[c0 + b];
-          const float dx = t.x.x - xj.x, dy = t.x.y - xj.y, dz = t.x.z - xj.z;
-          const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-          mask |= (d2 > wide ? 0u : 1u) << b;
+          const float rs = __fmaf_rn(xj.w, 1.00005f, rcm);
+          far = push_far(far, reach_left(__fmul_rn(rs, rs), sub3(t.x, f3(xj))));
         }
+        unsigned mask = near_mask(far, cn);
         const unsigned self = (unsigned)(i - c0);
         if (self < 32u) mask &= ~(1u << self);
         while (mask) {
-          const int j = c0 + __ffs(mask) - 1;
+          push(c0 + __ffs(mask) - 1);
           mask &= mask - 1u;
-          const float4 xj = a.xs[j];
-          const float dx = t.x.x - xj.x, dy = t.x.y - xj.y, dz = t.x.z - xj.z;
-          const float rs = rcs + xj.w;
-          const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-          if (!(d2 > rs * rs * 1.0001f)) push(j);
         }
       }
     };
