@@ -1142,6 +1142,7 @@ __global__ void k_compact(CompactArgs a) {
 }
 
 __global__ void k_adapt_counts(DevScalars* s, int n, int cap) {
+  pdl_wait(0);
   const int kept = s->n_kept;
   const int split = s->n_split;
   const int room = cap - kept;
@@ -1194,7 +1195,7 @@ gg_status split_and_compact(gg_system* S, cudaStream_t st) {
   a.remove_o = G.remove[o];
   auto kcomp = S->P.math_mode ? k_compact<1> : k_compact<0>;
   kcomp<<<nb, 256, 0, st>>>(a);
-  k_adapt_counts<<<1, 1, 0, st>>>(S->scal, (int)S->n, (int)S->cap);
+  GG_CUDA(launch_chained(k_adapt_counts, 1, 1, st, S->scal, (int)S->n, (int)S->cap));
   count_launches(S, 2);
   prof_end(S, PC_COMPACT, S->n, st);
   // the caller switches to the other buffers once it has read the counts
