@@ -428,6 +428,8 @@ __device__ __forceinline__ void up_finish(const UpArgs& a, int i, float4 p4, flo
 // candidate some lane hits.
 // 6 resident blocks of 256 (40 registers, no spills): the kernel is bound by
 // instruction issue, and 48 warps per SM hide its load latency better than 40.
+// It runs where k_upsample_pairs does not: supports shorter than a cell, and
+// systems without contact lists, whose memory holds the pairs.
 //
 // ALL: the support reaches every candidate of the stencil (a candidate lies
 // within 2 cell lengths of the point along each axis, so within sqrt(12) L,
@@ -503,6 +505,10 @@ __global__ void __launch_bounds__(256, 6) k_upsample(UpArgs a) {
 // no part either.  Against its marks, which leave each lane of a warp other
 // hits to gather: box scene (2.5 M points) 0.48 and 0.44 ms, settled pile
 // 0.46 and 0.26 ms, 1 M column with scaled constants 1.23 and 1.06 ms.
+//
+// Other shapes measured the same or slower (33.5 M points 9.31 ms, box scene
+// 0.436): 3 blocks of 256 with the loop unrolled by 4 9.30 and 0.478, 5 with
+// no unrolling 10.1 and 0.472, 8 blocks of 128 9.30 and 0.423.
 template <bool kCut>
 __global__ void __launch_bounds__(256, 4) k_upsample_pairs(UpArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
