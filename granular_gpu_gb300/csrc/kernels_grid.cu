@@ -607,17 +607,24 @@ __global__ void k_reorder_granular(int n, const uint32_t* perm,
                                    const int32_t* als_in, int32_t* als_out) {
   const int p = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   if (p >= n) return;
-  als_out[p] = als_in[p];  // stays where it is
+  // every load first: without __restrict__ (pdl_wait) a load does not move
+  // ahead of a store, and each would wait for the one before it.  8.4 M
+  // particles 0.169 ms with a plain launch, 0.222 field by field, 0.164 this way.
+  const int32_t als = als_in[p];  // stays where it is
   const uint32_t s = perm[p];
-  pos_out[p] = pos_in[s];
-  vel_out[p] = vel_in[s];
-  mass_out[p] = mass_in[s];
-  rs_out[p] = rs_in[s];
-  units_out[p] = units_in[s];
-  merge_out[p] = merge_in[s];
-  mu_out[p] = mu_in[s];
-  mc_out[p] = mc_in[s];
-  rm_out[p] = rm_in[s];
+  const float4 pos = pos_in[s], vel = vel_in[s];
+  const float mass = mass_in[s], rs = rs_in[s], merge = merge_in[s];
+  const int32_t units = units_in[s], mu = mu_in[s], mc = mc_in[s], rm = rm_in[s];
+  als_out[p] = als;
+  pos_out[p] = pos;
+  vel_out[p] = vel;
+  mass_out[p] = mass;
+  rs_out[p] = rs;
+  units_out[p] = units;
+  merge_out[p] = merge;
+  mu_out[p] = mu;
+  mc_out[p] = mc;
+  rm_out[p] = rm;
 }
 
 gg_status reorder_granular(gg_system* S, cudaStream_t st) {
@@ -642,8 +649,11 @@ __global__ void k_gather2(int n, const uint32_t* perm, const float4* a_in,
   const int p = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   if (p >= n) return;
   const uint32_t s = perm[p];
-  a_out[p] = a_in[s];
-  if (b_in) b_out[p] = b_in[s];
+  const float4 a = a_in[s];  // (both loads first, as in k_reorder_granular)
+  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (b_in) b = b_in[s];
+  a_out[p] = a;
+  if (b_in) b_out[p] = b;
 }
 
 __global__ void k_gather_boundary(int n, const uint32_t* __restrict__ perm, const float4* __restrict__ p_in,

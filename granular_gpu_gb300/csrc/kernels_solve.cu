@@ -49,14 +49,15 @@ __global__ void k_predict(int n, const float4* pos, const float4* vel,
   const int i = blockIdx.x * blockDim.x + (int)pdl_wait(threadIdx.x);
   unsigned int rbits = 0, dbits = 0;
   if (i < n) {
-    if (pn) pn[i] = 0.0f;
     const float4 p = pos[i];
     const float4 v4 = vel[i];
+    const float m = mass[i];  // (loads before stores: no pointer here is __restrict__)
     const float3 v = add3(f3(v4), dv);
     const float4 x = make_float4(p.x + dt * v.x, p.y + dt * v.y, p.z + dt * v.z, p.w);
     xs[i] = x;
-    const float sm = mass[i] * m_exp<MM>(-p.y);
+    const float sm = m * m_exp<MM>(-p.y);
     inv_m[i] = 1.0f / sm;
+    if (pn) pn[i] = 0.0f;
     rbits = __float_as_uint(fabsf(p.w));
     dbits = __float_as_uint(fmaxf(fmaxf(fabsf(x.x - p.x), fabsf(x.y - p.y)), fabsf(x.z - p.z)));
   }
