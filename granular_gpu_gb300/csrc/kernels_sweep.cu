@@ -70,7 +70,7 @@ struct SweepArgsT<true> {
   int long_rows;
   size_t li_row, li_step;  // entry k of particle i's list: nl_idx[i * li_row + k * li_step]
   const uint32_t* __restrict__ cell_inc;  // the last sweep's increments
-  uint32_t* __restrict__ cell_clear;  // the table of this sweep's, to be cleared (two take turns)
+  uint32_t* __restrict__ cell_clear;  // the table of this sweep's, to be cleared (two take turns), or null
   ResidualSlot* __restrict__ res;  // residual mode: this sweep's penetrations (kernels with bit 2 of MM)
   int count_builds;  // profiling: count the lists built
   int group_queue;  // queues up to this length are rebuilt by groups
@@ -617,11 +617,11 @@ __device__ __forceinline__ void apply_entries(const Args& a, const Target& t, in
   }
 }
 
-// Clears the table that the apply kernel of this sweep adds to (before a
-// plain launch it is cleared by its own).
+// Clears the table that the apply kernel of this sweep adds to (null where a
+// memset does: kClearPer).
 template <class Args>
 __device__ __forceinline__ void clear_increments(const Args& a, int tid) {
-  if (!std::is_same<Args, SweepArgs>::value) return;
+  if (!std::is_same<Args, SweepArgs>::value || !a.cell_clear) return;
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + tid; c <= a.g.C; c += (int64_t)gridDim.x * blockDim.x)
     a.cell_clear[c] = 0u;
 }
@@ -1198,6 +1198,21 @@ constexpr int64_t kGroupMax = 100000;
 // particles 5.5 against 5.7 ms, 144,000 5.1 against 4.4 ms).
 constexpr int64_t kChainMax = 400000;
 
+// The sweep's threads clear the increment table for its apply kernel where
+// that leaves each at most this many entries; a few particles in a large grid
+// leave it to a memset, which has the whole chip (and costs a launch, about
+// 3 us a sweep).  Substeps of 7 sweeps, by the threads and by memset: 300
+// particles in 1 M cells 122 and 134 us, 10 M 268 and 210, 100 M 1,654 and
+// 896; 4,000 in 100 M 948 and 957, 512 M 4,203 and 3,972; 120,000 (a thread
+// each) in 33 M 746 and 768, 100 M 1,310 and 1,265.
+constexpr int64_t kClearPer = 512;
+static gg_status clear_by_memset(gg_system* S, SweepArgs& a, int64_t threads, cudaStream_t st) {
+  if ((int64_t)S->grid.C + 1 <= kClearPer * threads) return GG_OK;
+  GG_CUDA(cudaMemsetAsync(a.cell_clear, 0, sizeof(uint32_t) * ((size_t)S->grid.C + 1), st));
+  a.cell_clear = nullptr;
+  return GG_OK;
+}
+
 // Queues up to this length are rebuilt by groups (30,000 to 240,000 measured
 // the same; 15,000 lost 30 % on 643,000 settled particles).
 constexpr int kGroupQueue = 65536;
@@ -1223,9 +1238,13 @@ constexpr int64_t kGroup32Max = 4096, kGroup16Max = 16384;
   }()
 
 template <int G>
-static void launch_group(const SweepArgs& a, int mm, cudaStream_t st) {
+static gg_status launch_group(gg_system* S, SweepArgs& a, int mm, cudaStream_t st) {
+  const int blocks = blocks_for(a.n, kGroupThreads / G);
+  gg_status rc = clear_by_memset(S, a, (int64_t)blocks * kGroupThreads, st);
+  if (rc != GG_OK) return rc;
   auto kern = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, G>);
-  launch_chained(kern, blocks_for(a.n, kGroupThreads / G), kGroupThreads, st, a);
+  GG_CUDA(launch_chained(kern, blocks, kGroupThreads, st, a));
+  return GG_OK;
 }
 
 static SweepArgsRO restricted(const SweepArgs& a) {
@@ -1299,16 +1318,18 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
   } else if (S->g.nl_idx && S->n <= kGroupMax) {
     a.li_row = kNlistMax;
     a.li_step = 1;
-    if (S->n <= kGroup32Max) launch_group<32>(a, mm, st);
-    else if (S->n <= kGroup16Max) launch_group<16>(a, mm, st);
-    else launch_group<8>(a, mm, st);
+    gg_status rc = S->n <= kGroup32Max   ? launch_group<32>(S, a, mm, st)
+                   : S->n <= kGroup16Max ? launch_group<16>(S, a, mm, st)
+                                         : launch_group<8>(S, a, mm, st);
+    if (rc != GG_OK) return rc;
   } else if (S->g.nl_idx) {
     a.li_row = 1;
     a.li_step = (size_t)S->cap;
     a.group_queue = kGroupQueue;
     const bool chain = S->n <= kChainMax;
+    gg_status rc = clear_by_memset(S, a, chain ? S->n : 0, st);
+    if (rc != GG_OK) return rc;
     const SweepArgsRO ro = restricted(a);
-    if (!chain) GG_CUDA(cudaMemsetAsync(a.cell_clear, 0, sizeof(uint32_t) * ((size_t)S->grid.C + 1), st));
     auto launch = [&](auto chained, auto plain, int blocks, int threads, auto... args) {
       if (chain) launch_chained(chained, blocks, threads, st, a, args...);
       else plain<<<blocks, threads, 0, st>>>(ro, args...);
