@@ -56,7 +56,7 @@ struct DevScalars {
   unsigned int disp0_bits;     // max |dt v| of the predict (float bits)
   unsigned int tile_fallback;  // sweep blocks that could not use the shared-memory tile
   int nl_queued[kMaxSweeps];          // per sweep: particles whose contact list is rebuilt
-  int nl_over;                 // long contact lists handed out in this substep
+  int nl_over;                 // particles that asked for a long contact list in this substep
   ResidualSlot res[kMaxSweeps];  // residual mode, per sweep
   int res_done;                // residual mode: 1 + the sweep whose x* met the target (later sweeps do nothing)
   unsigned int pen_bits;       // residual mode: largest penetration (float bits)

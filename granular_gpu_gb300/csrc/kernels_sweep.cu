@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kWarpThreads) k_sweep_list(SweepArgsRO a) {
 // nl_meta[i].w: the list's length, with flags when it holds walls and when it
 // is a long one; or why there is none.  From kNlistLong up it is the groups'.
 constexpr int kNlistWalls = 1 << 16, kNlistLong = 1 << 17, kNlistCount = kNlistWalls - 1;
-constexpr int kNlistNone = 1 << 18;  // too many for a long one (or all are taken): the groups scan every sweep
+constexpr int kNlistNone = 1 << 18;  // too many for its long one (or all are taken): the groups scan every sweep
 constexpr int kNlistNew = -1;        // too many candidates for a list of kNlistMax: the groups make a long one
 constexpr int kNlistAgain = -2;      // the same, found in a short queue: queued again at the next sweep
 
@@ -915,12 +915,14 @@ __device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* 
   make_target_lite(a, is, a.xs[is], t);
   int cnt = 0;
   bool walls = false, rebuild = act, counted = true;
-  // the long list, and where this one is: -1 none yet, -2 none to be had
+  // the particle's long list: -1 none yet, -2 none to be had.  Once it has one
+  // it keeps it, through sweeps whose candidates it does not hold as well
+  // (row[0] remembers which).
   int long_row = kWork == kWorkAll ? -1 : kWork == kWorkLong && slot < a.long_rows ? slot : -2;
   int32_t* row = a.nl_idx + is * a.li_row;
   if (kWork == kWorkLong || (kWork == kWorkAll && a.it > 0)) {
     const int4 m = a.nl_meta[is];
-    if (kWork == kWorkAll && m.w >= 0 && (m.w & kNlistLong)) long_row = row[0];
+    if (kWork == kWorkAll && m.w >= 0 && (m.w & (kNlistLong | kNlistNone))) long_row = row[0];
     counted = m.w != kNlistNew;  // (the threads that left it counted it)
     const bool same = act && m.w >= 0 && m.w != kNlistNone && m.x == t.q.x && m.y == t.q.y && m.z == t.q.z;
     const float A0 = a.nl_acc[is];
@@ -959,8 +961,8 @@ __device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* 
   __syncwarp();
   const float Bs = t.Bf + a.skin, Bs2 = Bs * Bs * 1.0001f;
   const float rcs = t.rc + a.skin;
-  bool over = false;
-  int stored = 0;  // entries in the long list
+  bool over = false, fits = true;
+  int stored = 0;  // entries for the long list, which it holds if it fits
   float sum = 0.0f;  // component gl of the corrections
   int c = 0, s_loc = 0;
   // the scan's place (the same for all groups of a warp): column and cell,
@@ -1046,8 +1048,8 @@ __device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* 
     if (rebuild && (filled || done)) {
       // (a particle that has a long list keeps to it)
       if (over || long_row >= 0) {
-        if (stored + cnt > kLongMax) long_row = -2;
-        if (long_row >= 0)
+        fits &= stored + cnt <= kLongMax;
+        if (long_row >= 0 && fits)
           for (int k = gl; k < cnt; k += G) a.nl_long[(size_t)long_row * kLongMax + stored + k] = s_list[grp][k];
         stored += cnt;
       } else {
@@ -1055,12 +1057,9 @@ __device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* 
       }
       if (done && gl == 0) {
         int w = cnt;
-        if (long_row >= 0) {
-          w = stored | kNlistLong;
-          if (kWork == kWorkAll) row[0] = long_row;
-        } else if (over || kWork == kWorkLong) {
-          w = kWork == kWorkQueue ? kNlistAgain : kNlistNone;
-        }
+        if (long_row >= 0 && fits) w = stored | kNlistLong;
+        else if (over || kWork == kWorkLong) w = kWork == kWorkQueue ? kNlistAgain : kNlistNone;
+        if (kWork == kWorkAll && w >= kNlistLong) row[0] = long_row;
         if (walls && w >= 0 && w != kNlistNone) w |= kNlistWalls;
         a.nl_meta[i] = make_int4(t.q.x, t.q.y, t.q.z, w);
         a.nl_acc[i] = 0.0f;
