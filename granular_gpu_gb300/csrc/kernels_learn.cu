@@ -1210,6 +1210,12 @@ gg_status solve_to_residual(gg_system* S, int first, int cap, cudaStream_t st, i
       const int at = S->scal_host->res_done - 1;
       const ResidualSlot& r = S->scal_host->res[at];
       *sweeps = at - first;
+      if (S->profiling) {
+        // no units for what returned at once: the sweeps behind the one that
+        // met the target, and its apply
+        S->prof_units[PC_SWEEP] -= S->n * (k - *sweeps - 1);
+        S->prof_units[PC_APPLY] -= S->n * (k - *sweeps);
+      }
       *out = residual_mean(r.sum, r.count);
       std::memcpy(&S->last_residual_max, &r.most_bits, sizeof(float));
       return GG_OK;
