@@ -27,69 +27,19 @@
 // autotuner may pick where lists do not pay.
 #include <algorithm>
 #include <climits>
-#include <cstring>
 #include <type_traits>
 
 #include "common.cuh"
 
 namespace gg {
 
-// The arguments of the sweep kernels, with pointers that are __restrict__
-// (SweepArgsRO, for kernels launched plainly: loads may take the read-only
-// path and move across stores) or not (SweepArgs, for kernels launched
-// chained).  Same fields, same layout.
-template <bool kRestrict>
-struct SweepArgsT;
-template <>
-struct SweepArgsT<true> {
-  Grid g;
-  int n;
-  int it;
-  const float4* __restrict__ xs;
-  const float* __restrict__ inv_m;
-  const uint32_t* __restrict__ keys;
-  const int32_t* __restrict__ cs;
-  const int32_t* __restrict__ bcs;
-  const float4* __restrict__ bpos;
-  float4* __restrict__ delta;
-  int32_t* __restrict__ s_extra;
-  DevScalars* __restrict__ scal;
-  double brad;  // boundary radius (double literal 0.01)
-  double fcap;  // friction cap (double literal 0.8)
-  float fcapf;  // the same as float
-  float bradf;  // brad as float (conservative cuts only)
-  const float2* __restrict__ window;  // per cell coordinate: positions whose query cell is within one of it
-  float minr;  // floor of the particle radius against walls (0.01f)
-  // contact candidate lists (the default sweep)
-  int32_t* __restrict__ nl_idx;
-  int4* __restrict__ nl_meta;
-  float* __restrict__ nl_acc;
-  int32_t* __restrict__ nl_queue;
-  int32_t* __restrict__ nl_over;  // particles with long lists, left to the groups
-  int32_t* __restrict__ nl_long;  // the long lists, kLongMax entries each
-  int long_rows;
-  size_t li_row, li_step;  // entry k of particle i's list: nl_idx[i * li_row + k * li_step]
-  const uint32_t* __restrict__ cell_inc;  // the last sweep's increments
-  uint32_t* __restrict__ cell_clear;  // the table of this sweep's, to be cleared (two take turns), or null
-  ResidualSlot* __restrict__ res;  // residual mode: this sweep's penetrations (kernels with bit 2 of MM)
-  int count_builds;  // profiling: count the lists built
-  int group_queue;  // queues up to this length are rebuilt by groups
-  float skin;
-  float eabs;  // bound on the rounding of one position update
-  UDiv div_yz, div_z;  // division by ny * nz and by nz (binning cell of a key)
-  // batched scenes: scene of a particle = its x* slab, floor(x / width);
-  // each scene has its own friction cap (null: a.fcap for every particle)
-  const float* __restrict__ scene_fcap;
-  float scene_inv_w;
-  int n_scenes;
-  // configured mode (gg_params.contact_law): substep-start positions for
-  // the friction law and its output, the summed friction corrections and
-  // their count (both null with the reference's law)
-  const float4* __restrict__ pos0;
-  float4* __restrict__ fdelta;
-};
-template <>
-struct SweepArgsT<false> {
+// The arguments of the sweep kernels.  No pointer is __restrict__: the kernels
+// with contact lists are launched chained (pdl_wait), at every size.  Against
+// plain launches with __restrict__ above 400,000 particles: the 8.4 M column
+// 28.5 to 28.0 ms a substep, a batch of 643,000 4.52 to 4.37 for two, 8 M
+// particles falling free of each other 4.21 and 4.31.  The kernels without
+// lists measured the same either way.
+struct SweepArgs {
   Grid g;
   int n;
   int it;
@@ -102,44 +52,40 @@ struct SweepArgsT<false> {
   float4* delta;
   int32_t* s_extra;
   DevScalars* scal;
-  double brad;
-  double fcap;
-  float fcapf;
-  float bradf;
-  const float2* window;
-  float minr;
+  double brad;  // boundary radius (double literal 0.01)
+  double fcap;  // friction cap (double literal 0.8)
+  float fcapf;  // the same as float
+  float bradf;  // brad as float (conservative cuts only)
+  const float2* window;  // per cell coordinate: positions whose query cell is within one of it
+  float minr;  // floor of the particle radius against walls (0.01f)
+  // contact candidate lists (the default sweep)
   int32_t* nl_idx;
   int4* nl_meta;
   float* nl_acc;
   int32_t* nl_queue;
-  int32_t* nl_over;
-  int32_t* nl_long;
+  int32_t* nl_over;  // particles with long lists, left to the groups
+  int32_t* nl_long;  // the long lists, kLongMax entries each
   int long_rows;
-  size_t li_row, li_step;
-  const uint32_t* cell_inc;
-  uint32_t* cell_clear;
-  ResidualSlot* res;
-  int count_builds;
-  int group_queue;
+  size_t li_row, li_step;  // entry k of particle i's list: nl_idx[i * li_row + k * li_step]
+  const uint32_t* cell_inc;  // the last sweep's increments
+  uint32_t* cell_clear;  // the table of this sweep's, to be cleared (two take turns), or null
+  ResidualSlot* res;  // residual mode: this sweep's penetrations (kernels with bit 2 of MM)
+  int count_builds;  // profiling: count the lists built
+  int group_queue;  // queues up to this length are rebuilt by groups
   float skin;
-  float eabs;
-  UDiv div_yz, div_z;
+  float eabs;  // bound on the rounding of one position update
+  UDiv div_yz, div_z;  // division by ny * nz and by nz (binning cell of a key)
+  // batched scenes: scene of a particle = its x* slab, floor(x / width);
+  // each scene has its own friction cap (null: a.fcap for every particle)
   const float* scene_fcap;
   float scene_inv_w;
   int n_scenes;
+  // configured mode (gg_params.contact_law): substep-start positions for
+  // the friction law and its output, the summed friction corrections and
+  // their count (both null with the reference's law)
   const float4* pos0;
   float4* fdelta;
 };
-using SweepArgs = SweepArgsT<false>;
-using SweepArgsRO = SweepArgsT<true>;
-static_assert(sizeof(SweepArgs) == sizeof(SweepArgsRO), "one layout");
-
-// The thread index, after the wait of a chained launch (a plain one keeps
-// the hardware's, which costs no register).
-template <class Args>
-__device__ __forceinline__ int sweep_thread() {
-  return std::is_same<Args, SweepArgs>::value ? (int)pdl_wait(threadIdx.x) : (int)threadIdx.x;
-}
 
 // The kernels' template argument MM: bit 0 the math mode (0 CUDA's
 // functions, 1 rounded once from double), bit 1 the contact law (0 the
@@ -186,28 +132,24 @@ struct Share {
 
 // The friction cap in double, as the reference's comparisons and ratios use
 // it (rare paths only, so targets carry the float copy).
-template <class Args>
-__device__ __forceinline__ double target_fcap(const Args& a, const Target& t) {
+__device__ __forceinline__ double target_fcap(const SweepArgs& a, const Target& t) {
   if (!a.scene_fcap) return a.fcap;
   const int s = min(max(__float2int_rz(t.x.x * a.scene_inv_w), 0), a.n_scenes - 1);
   return (double)a.scene_fcap[s];
 }
 // 0.01 + r_b in double (Solver.cu:283).
-template <class Args>
-__device__ __forceinline__ double target_bd(const Args& a, const Target& t) { return a.brad + (double)t.rb; }
+__device__ __forceinline__ double target_bd(const SweepArgs& a, const Target& t) { return a.brad + (double)t.rb; }
 
 // The thresholds of the wall contacts, in double; needed only by targets
 // with walls in reach (FP64 issues at 1/64 of the FP32 rate).
-template <class Args>
-__device__ __forceinline__ void target_walls(const Args& a, Target& t) {
+__device__ __forceinline__ void target_walls(const SweepArgs& a, Target& t) {
   t.Bru = __double2float_ru(target_bd(a, t));
   t.capBru = __double2float_ru(((double)t.rb + a.brad) * target_fcap(a, t));
 }
 
 // The per-target values every sweep needs (no pruning masks, no wall
 // thresholds).
-template <class Args>
-__device__ __forceinline__ void make_target_lite(const Args& a, int i, float4 xi4, Target& t) {
+__device__ __forceinline__ void make_target_lite(const SweepArgs& a, int i, float4 xi4, Target& t) {
   const Grid& g = a.g;
   t.x = f3(xi4);
   t.rc = xi4.w;
@@ -233,8 +175,7 @@ __device__ __forceinline__ void make_target_lite(const Args& a, int i, float4 xi
 
 // Pruning masks: the stencil columns that can hold a partner within
 // r_i + r_max plus the displacement since binning, or a wall within reach.
-template <class Args>
-__device__ __forceinline__ void target_masks(const Args& a, Target& t) {
+__device__ __forceinline__ void target_masks(const SweepArgs& a, Target& t) {
   const Grid& g = a.g;
   float disp = __uint_as_float(a.scal->disp0_bits);
   for (int k = 0; k < a.it; ++k) disp += __uint_as_float(a.scal->inc_bits[k]);
@@ -251,8 +192,7 @@ __device__ __forceinline__ void target_masks(const Args& a, Target& t) {
   t.bm[2] = axis_mask(t.x.z, t.q.z, g.L, Rb);
 }
 
-template <class Args>
-__device__ __forceinline__ void make_target(const Args& a, int i, float4 xi4, Target& t) {
+__device__ __forceinline__ void make_target(const SweepArgs& a, int i, float4 xi4, Target& t) {
   make_target_lite(a, i, xi4, t);
   target_walls(a, t);
   target_masks(a, t);
@@ -263,8 +203,8 @@ __device__ __forceinline__ void make_target(const Args& a, int i, float4 xi4, Ta
 // compares below a double D exactly when it compares below D rounded up to
 // float (no float lies strictly between the two roundings of D), so the
 // double comparisons are decided in float.
-template <int MM, class Args>
-__device__ __forceinline__ bool wall_contact(const Args& a, const Target& t, float4 pb, Share& s) {
+template <int MM>
+__device__ __forceinline__ bool wall_contact(const SweepArgs& a, const Target& t, float4 pb, Share& s) {
   const float bx = t.x.x - pb.x, by = t.x.y - pb.y, bz = t.x.z - pb.z;
   const float dis = m_norm3<(MM & 1)>(bx, by, bz);
   if (!(dis < t.Bru)) return false;  // mag < 0
@@ -302,8 +242,8 @@ __device__ __forceinline__ bool wall_near(const Target& t, float4 pb) {
 // particles_constraint for one candidate j (Solver.cu:314-357): whether it
 // is a contact, its share, and whether j finds the target too (else the
 // count is handed to j here).
-template <int MM, class Args>
-__device__ __forceinline__ bool pair_contact(const Args& a, const Target& t, int j, float4 xj4, float inv_mj,
+template <int MM>
+__device__ __forceinline__ bool pair_contact(const SweepArgs& a, const Target& t, int j, float4 xj4, float inv_mj,
                                              Share& s, bool& back) {
   back = false;
   const float dx = t.x.x - xj4.x, dy = t.x.y - xj4.y, dz = t.x.z - xj4.z;
@@ -380,8 +320,7 @@ __device__ __forceinline__ void add_penetration(const Target& t, int e, float4 p
   }
 }
 // A block's penetrations into its sweep's slot (every thread calls it).
-template <class Args>
-__device__ __forceinline__ void store_penetration(const Args& a, const Penetration& u) {
+__device__ __forceinline__ void store_penetration(const SweepArgs& a, const Penetration& u) {
   __shared__ float s_sum[8];
   __shared__ unsigned int s_count[8], s_most[8];
   float ws = u.sum;
@@ -417,16 +356,16 @@ struct Sums {
   float3 dp = {0.f, 0.f, 0.f}, df = {0.f, 0.f, 0.f};
   int c = 0, s_loc = 0;
 };
-template <int MM, class Args>
-__device__ __forceinline__ void add_wall(const Args& a, const Target& t, float4 pb, Sums& u) {
+template <int MM>
+__device__ __forceinline__ void add_wall(const SweepArgs& a, const Target& t, float4 pb, Sums& u) {
   Share s;
   if (!wall_contact<MM>(a, t, pb, s)) return;
   u.dp = add3(u.dp, s.dp);
   if (MM & 2) u.df = add3(u.df, s.df);
   ++u.c;
 }
-template <int MM, class Args>
-__device__ __forceinline__ void add_pair(const Args& a, const Target& t, int j, float4 xj4, float inv_mj, Sums& u) {
+template <int MM>
+__device__ __forceinline__ void add_pair(const SweepArgs& a, const Target& t, int j, float4 xj4, float inv_mj, Sums& u) {
   Share s;
   bool back;
   if (!pair_contact<MM>(a, t, j, xj4, inv_mj, s, back)) return;
@@ -435,8 +374,8 @@ __device__ __forceinline__ void add_pair(const Args& a, const Target& t, int j, 
   ++u.c;
   if (back) ++u.s_loc;
 }
-template <int MM, class Args>
-__device__ __forceinline__ void store_sums(const Args& a, int i, const Sums& u) {
+template <int MM>
+__device__ __forceinline__ void store_sums(const SweepArgs& a, int i, const Sums& u) {
   a.delta[i] = make_float4(u.dp.x, u.dp.y, u.dp.z, __int_as_float((u.c & 0xffff) | (u.s_loc << 16)));
   // (every contact emits one friction target, so their count is c)
   if (MM & 2) a.fdelta[i] = make_float4(u.df.x, u.df.y, u.df.z, __int_as_float(u.c));
@@ -447,8 +386,8 @@ __device__ __forceinline__ bool use_cell(const unsigned* m, int ox, int oy, int 
 }
 
 // The reference loop for one target over global memory.
-template <int MM, class Args>
-__device__ void sweep_global(const Args& a, int i, const Target& t) {
+template <int MM>
+__device__ void sweep_global(const SweepArgs& a, int i, const Target& t) {
   const Grid& g = a.g;
   Sums u;
   for (int ox = 0; ox < 3; ++ox) {
@@ -479,7 +418,7 @@ __device__ void sweep_global(const Args& a, int i, const Target& t) {
 }
 
 template <int MM>
-__global__ void __launch_bounds__(256) k_sweep(SweepArgsRO a) {
+__global__ void __launch_bounds__(256) k_sweep(SweepArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   Target t;
@@ -500,8 +439,8 @@ __global__ void __launch_bounds__(256) k_sweep(SweepArgsRO a) {
 constexpr int kWarpList = 32;      // listed candidates per lane before a flush
 constexpr int kWarpThreads = 256;
 
-template <int MM, class Args>
-__device__ __forceinline__ void process_entry(const Args& a, const Target& t, int e, Sums& u) {
+template <int MM>
+__device__ __forceinline__ void process_entry(const SweepArgs& a, const Target& t, int e, Sums& u) {
   if (e < 0) add_wall<MM>(a, t, a.bpos[-e - 1], u);
   else add_pair<MM>(a, t, e, a.xs[e], a.inv_m[e], u);
 }
@@ -511,7 +450,7 @@ __device__ __forceinline__ void process_entry(const Args& a, const Target& t, in
 // pass the cheap distance test listed in order and processed by all lanes
 // together afterwards.
 template <int MM>
-__global__ void __launch_bounds__(kWarpThreads) k_sweep_list(SweepArgsRO a) {
+__global__ void __launch_bounds__(kWarpThreads) k_sweep_list(SweepArgs a) {
   __shared__ int s_list[kWarpThreads / 32][kWarpList][32];
   const Grid& g = a.g;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -585,8 +524,7 @@ constexpr int kNlistAgain = -2;      // the same, found in a short queue: queued
 // The listed candidates in order, with the next entry's gathers issued
 // before the current one is processed.  entry(k) gives the k-th entry: a
 // particle index, or -(wall index) - 1.
-template <class Args>
-__device__ __forceinline__ void fetch_entry(const Args& a, int e, float4& p, float& im) {
+__device__ __forceinline__ void fetch_entry(const SweepArgs& a, int e, float4& p, float& im) {
   if (e >= 0) {
     p = a.xs[e];
     im = a.inv_m[e];
@@ -595,8 +533,8 @@ __device__ __forceinline__ void fetch_entry(const Args& a, int e, float4& p, flo
   }
 }
 
-template <int MM, class Args, class EntryF>
-__device__ __forceinline__ void apply_entries(const Args& a, const Target& t, int cnt, EntryF&& entry,
+template <int MM, class EntryF>
+__device__ __forceinline__ void apply_entries(const SweepArgs& a, const Target& t, int cnt, EntryF&& entry,
                                               Sums& u, Penetration& pen) {
   if (cnt <= 0) return;
   int e_next = entry(0);
@@ -619,21 +557,18 @@ __device__ __forceinline__ void apply_entries(const Args& a, const Target& t, in
 
 // Clears the table that the apply kernel of this sweep adds to (null where a
 // memset does: kClearPer).
-template <class Args>
-__device__ __forceinline__ void clear_increments(const Args& a, int tid) {
-  if (!std::is_same<Args, SweepArgs>::value || !a.cell_clear) return;
+__device__ __forceinline__ void clear_increments(const SweepArgs& a, int tid) {
+  if (!a.cell_clear) return;
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + tid; c <= a.g.C; c += (int64_t)gridDim.x * blockDim.x)
     a.cell_clear[c] = 0u;
 }
 
-template <class Args>
-__device__ __forceinline__ bool nlist_bound_ok(const Args& a, float A) {
+__device__ __forceinline__ bool nlist_bound_ok(const SweepArgs& a, float A) {
   return A * 1.0001f + 4.0f * a.eabs < a.skin;
 }
 
 // One sweep's share of the bound A for an increment-length bound N.
-template <class Args>
-__device__ __forceinline__ float nlist_step(const Args& a, float N) { return 2.0f * (N + 1.7320509f * a.eabs); }
+__device__ __forceinline__ float nlist_step(const SweepArgs& a, float N) { return 2.0f * (N + 1.7320509f * a.eabs); }
 
 // Largest per-cell increment of the last sweep over the stencil of q and the
 // particle's own binning cell.  Every cell_inc entry holds the largest
@@ -642,8 +577,7 @@ __device__ __forceinline__ float nlist_step(const Args& a, float N) { return 2.0
 // the own cell adds its entry when it is not one of the 27 (the entry bounds
 // its increment from above).  A query cell outside the grid in z reads the
 // stencil's cells one by one (entries that may bound from above as well).
-template <class Args>
-__device__ __forceinline__ float nlist_cell_bound(const Args& a, int3 q, uint32_t own_key) {
+__device__ __forceinline__ float nlist_cell_bound(const SweepArgs& a, int3 q, uint32_t own_key) {
   const Grid& g = a.g;
   uint32_t m = 0u;
   if (q.z >= 0 && q.z < g.nz) {
@@ -674,13 +608,14 @@ __device__ __forceinline__ float nlist_cell_bound(const Args& a, int3 q, uint32_
 
 // Sweeps after the first: particles whose list is still exact run it; the
 // others are queued for k_sweep_nlist_build.
-// 5 resident blocks of 256 (48 registers; the per-target state carries no
-// double, and a few bytes spill): about 2 % faster than 4 blocks at 64 in the
-// large systems that are launched plainly.
-template <int MM, class Args>
-__global__ void __launch_bounds__(256, std::is_same<Args, SweepArgs>::value ? 4 : 5) k_sweep_nlist_keep(Args a) {
+// 4 resident blocks of 256 (64 registers): substeps of the 8.4 M column 28.3 ms
+// against 28.6 with 5 (48 registers), batch of 643,000 4.40 and 4.57, warm-started
+// 144,000 4.33 and 4.66; 8 M particles falling free of each other, whose lists
+// are empty, 4.44 and 4.26.
+template <int MM>
+__global__ void __launch_bounds__(256, 4) k_sweep_nlist_keep(SweepArgs a) {
   const Grid& g = a.g;
-  const int tid = sweep_thread<Args>();
+  const int tid = (int)pdl_wait(threadIdx.x);
   if ((MM & 4) && a.scal->res_done) return;
   clear_increments(a, tid);
   const int i = blockIdx.x * blockDim.x + tid;
@@ -742,10 +677,10 @@ constexpr int kBuildThreads = 128;
 
 // 8 resident blocks of 128 (64 registers): the rebuilds are latency-bound
 // (72 registers and 7 blocks measured 3 % slower over the sweeps).
-template <int MM, class Args>
-__global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(Args a, int queued) {
+template <int MM>
+__global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArgs a, int queued) {
   const Grid& g = a.g;
-  const int tid = sweep_thread<Args>(), lane = tid & 31;
+  const int tid = (int)pdl_wait(threadIdx.x), lane = tid & 31;
   const int total = queued ? a.scal->nl_queued[a.it] : a.n;
   if (queued && total <= a.group_queue) return;  // the groups take a short queue
   if ((MM & 4) && a.scal->res_done) return;
@@ -1192,11 +1127,6 @@ gg_status window_table(gg_system* S, cudaStream_t st) {
 // the line lies where a thread to a particle starts to fill the chip.
 constexpr int64_t kGroupMax = 100000;
 
-// Systems up to this size launch the thread kernels chained; above it the
-// read-only path is worth more than the gaps between launches (643,000
-// particles 5.5 against 5.7 ms, 144,000 5.1 against 4.4 ms).
-constexpr int64_t kChainMax = 400000;
-
 // The sweep's threads clear the increment table for its apply kernel where
 // that leaves each at most this many entries; a few particles in a large grid
 // leave it to a memset, which has the whole chip (and costs a launch, about
@@ -1244,12 +1174,6 @@ static gg_status launch_group(gg_system* S, SweepArgs& a, int mm, cudaStream_t s
   auto kern = GG_SWEEP_KERNEL(mm, k_sweep_group<MM, G>);
   GG_CUDA(launch_chained(kern, blocks, kGroupThreads, st, a));
   return GG_OK;
-}
-
-static SweepArgsRO restricted(const SweepArgs& a) {
-  SweepArgsRO r;
-  std::memcpy(&r, &a, sizeof(r));
-  return r;
 }
 
 bool sweep_lists(const gg_system* S) { return S->g.nl_idx && S->tune.sweep_variant == 0; }
@@ -1313,7 +1237,7 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
   // one-thread-per-particle stencil sweep instead (same results)
   if (S->tune.sweep_variant == 1) {
     auto kern = (mm == 0 ? k_sweep<0> : mm == 1 ? k_sweep<1> : mm == 2 ? k_sweep<2> : k_sweep<3>);
-    kern<<<blocks_for(S->n, 256), 256, 0, st>>>(restricted(a));
+    kern<<<blocks_for(S->n, 256), 256, 0, st>>>(a);
   } else if (S->g.nl_idx && S->n <= kGroupMax) {
     a.li_row = kNlistMax;
     a.li_step = 1;
@@ -1325,34 +1249,26 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
     a.li_row = 1;
     a.li_step = (size_t)S->cap;
     a.group_queue = kGroupQueue;
-    const bool chain = S->n <= kChainMax;
-    gg_status rc = clear_by_memset(S, a, chain ? S->n : 0, st);
+    gg_status rc = clear_by_memset(S, a, S->n, st);
     if (rc != GG_OK) return rc;
-    const SweepArgsRO ro = restricted(a);
-    auto launch = [&](auto chained, auto plain, int blocks, int threads, auto... args) {
-      if (chain) launch_chained(chained, blocks, threads, st, a, args...);
-      else plain<<<blocks, threads, 0, st>>>(ro, args...);
-    };
-    auto build = GG_SWEEP_KERNEL(mm, k_sweep_nlist_build<MM, SweepArgs>);
-    auto build_ro = GG_SWEEP_KERNEL(mm, k_sweep_nlist_build<MM, SweepArgsRO>);
+    auto build = GG_SWEEP_KERNEL(mm, k_sweep_nlist_build<MM>);
     if (it == 0) {
-      launch(build, build_ro, blocks_for(S->n, kBuildThreads), kBuildThreads, 0);
+      GG_CUDA(launch_chained(build, blocks_for(S->n, kBuildThreads), kBuildThreads, st, a, 0));
     } else {
-      auto keep = GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM, SweepArgs>);
-      auto keep_ro = GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM, SweepArgsRO>);
+      auto keep = GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM>);
       const int tk = S->tune.keep_threads;
-      launch(keep, keep_ro, blocks_for(S->n, tk), tk);
+      GG_CUDA(launch_chained(keep, blocks_for(S->n, tk), tk, st, a));
       const int nb = std::min(blocks_for(S->n, kBuildThreads), S->num_sms * S->tune.build_blocks_per_sm);
-      launch(build, build_ro, nb, kBuildThreads, 1);
+      GG_CUDA(launch_chained(build, nb, kBuildThreads, st, a, 1));
       count_launches(S, 1);
     }
     // short queues, and what a list does not hold
     auto rest = GG_SWEEP_KERNEL(mm, k_sweep_rest<MM>);
-    launch_chained(rest, S->num_sms * 3, kGroupThreads, st, a);
+    GG_CUDA(launch_chained(rest, S->num_sms * 3, kGroupThreads, st, a));
     count_launches(S, 1);
   } else {
     auto kern = (mm == 0 ? k_sweep_list<0> : mm == 1 ? k_sweep_list<1> : mm == 2 ? k_sweep_list<2> : k_sweep_list<3>);
-    kern<<<blocks_for(S->n, kWarpThreads), kWarpThreads, 0, st>>>(restricted(a));
+    kern<<<blocks_for(S->n, kWarpThreads), kWarpThreads, 0, st>>>(a);
   }
   count_launches(S, 1);
   prof_end(S, PC_SWEEP, S->n, st);
