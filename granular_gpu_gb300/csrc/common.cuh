@@ -209,11 +209,14 @@ __host__ __device__ __forceinline__ float residual_mean(double sum, unsigned int
 // launched by launch_chained is set up on the chip while the one before it
 // in the stream ends, and its first pdl_wait returns once that one (and so
 // every one before it) has completed and its writes are visible.  Every
-// kernel launched this way calls pdl_wait before it touches memory, and
-// derives its addresses from the value that comes back (the thread index
-// that it is given), so that no load can be moved ahead of the wait; and none
-// of its loads takes the read-only path (no __restrict__ const pointer),
-// which may return what the cache held before.  Measured on a GB300 with the
+// kernel launched this way calls pdl_wait before it touches memory: a volatile
+// statement that clobbers memory, which no load or store moves ahead of as
+// long as its pointer is not const __restrict__ (such a load may also take the
+// read-only path, which may return what the cache held before), so none of
+// them has one.  The thread index is passed through as well, for the addresses
+// that depend on it; flags and counters at fixed addresses rest on the clobber
+// alone.  Without __restrict__ loads stay behind earlier stores, so kernels
+// load before they store.  Measured on a GB300 with the
 // clears and copies between the kernels folded into them: a frame of 4
 // substeps of 1,000 particles 776 to 486 us, a warm-started substep of 76
 // sweeps 6.1 to 4.3 ms, a grid build of 200,000 points 51 to 41 us.  (Letting the next kernel's
