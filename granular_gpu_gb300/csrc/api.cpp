@@ -670,7 +670,8 @@ gg_status gg_profile_begin(gg_system* S) {
   S->prof_pool_used = 0;
   S->prof_launch_base = S->launches;
   S->profiling = true;
-  if (cudaMemsetAsync(&S->scal->nlist_rebuilds, 0, sizeof(S->scal->nlist_rebuilds), S->stream) != cudaSuccess) {
+  if (cudaMemsetAsync(&S->scal->nlist_rebuilds, 0, sizeof(S->scal->nlist_rebuilds), S->stream) != cudaSuccess ||
+      cudaMemsetAsync(&S->scal->count_builds, 1, sizeof(S->scal->count_builds), S->stream) != cudaSuccess) {
     set_error("gg_profile_begin: cannot reset the device counters");
     return GG_ERR_CUDA;
   }
@@ -688,6 +689,7 @@ gg_status gg_profile_end(gg_system* S, gg_profile_t* out) {
   unsigned long long rebuilds = 0;
   if (cudaMemcpyAsync(&rebuilds, &S->scal->nlist_rebuilds, sizeof(rebuilds), cudaMemcpyDeviceToHost, S->stream) !=
           cudaSuccess ||
+      cudaMemsetAsync(&S->scal->count_builds, 0, sizeof(S->scal->count_builds), S->stream) != cudaSuccess ||
       cudaStreamSynchronize(S->stream) != cudaSuccess) {
     set_error("gg_profile_end: cannot read the device counters");
     return GG_ERR_CUDA;

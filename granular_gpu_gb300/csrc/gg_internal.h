@@ -71,6 +71,7 @@ struct DevScalars {
   int n_split_appended;
   int n_kept;
   unsigned long long nlist_rebuilds;  // listed-sweep list builds, counted while profiling (not reset per substep)
+  int count_builds;            // profiling (read by the kernels, which a graph may have captured before)
 };
 
 

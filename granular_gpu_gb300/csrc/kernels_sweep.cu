@@ -70,7 +70,6 @@ struct SweepArgs {
   const uint32_t* cell_inc;  // the last sweep's increments
   uint32_t* cell_clear;  // the table of this sweep's, to be cleared (two take turns), or null
   ResidualSlot* res;  // residual mode: this sweep's penetrations (kernels with bit 2 of MM)
-  int count_builds;  // profiling: count the lists built
   int group_queue;  // queues up to this length are rebuilt by groups
   float skin;
   float eabs;  // bound on the rounding of one position update
@@ -690,8 +689,11 @@ __global__ void __launch_bounds__(kBuildThreads, 8) k_sweep_nlist_build(SweepArg
     const int slot = base + tid;
     const bool act = slot < total;
     {
+      // (the vote also brings the warp back together: 8.4 M column 28.2 ms a
+      // substep, 28.5 with the vote inside the condition and a __syncwarp)
       const unsigned bal = __ballot_sync(0xffffffffu, act);
-      if (lane == 0 && bal) atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)__popc(bal));
+      if (a.scal->count_builds && lane == 0 && bal)
+        atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)__popc(bal));
     }
     if (!act) continue;
     const int i = queued ? a.nl_queue[slot] : slot;
@@ -825,6 +827,7 @@ __device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* 
   const Grid& g = a.g;
   const int lane = tid & 31, gl = lane & (G - 1), grp = tid / G;
   const unsigned glt = (1u << gl) - 1u;
+  const bool count = a.scal->count_builds != 0;
   auto gballot = [&](bool p) {
     const unsigned b = __ballot_sync(kAll, p);
     return G == 32 ? b : (b >> (lane & ~(G - 1))) & ((1u << (G & 31)) - 1u);
@@ -1047,7 +1050,7 @@ __device__ __forceinline__ void sweep_groups(const SweepArgs& a, int tid, void* 
       if (gl == 6) out[3] = __int_as_float(c);
     }
   }
-  if (a.count_builds) {
+  if (count) {
     const unsigned b = __ballot_sync(kAll, rebuild && counted && gl == 0);
     if (lane == 0 && b) atomicAdd(&a.scal->nlist_rebuilds, (unsigned long long)__popc(b));
   }
@@ -1221,7 +1224,6 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
   a.long_rows = (int)std::min<int64_t>(kLongInts * S->cap / kLongMax, INT_MAX);
   a.li_row = a.li_step = 0;
   a.group_queue = 0;
-  a.count_builds = S->profiling ? 1 : 0;
   a.skin = S->nl_skin;
   a.div_yz = make_udiv((uint32_t)(S->grid.ny * S->grid.nz));
   a.div_z = make_udiv((uint32_t)S->grid.nz);
