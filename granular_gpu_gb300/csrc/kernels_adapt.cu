@@ -203,14 +203,19 @@ __global__ void __launch_bounds__(kSurfThreads, 6) k_surface(SurfArgs a) {
 // to a component; the vote runs over the list again, or, where it did not
 // hold all of them, over the stencil.
 //
-// Measured on a GB300 (same bits), thread against group: 51,000 particles of
-// the box scene 0.118 and 0.045 ms, 125,000 of the settled pile 0.44 and
-// 0.34 ms, 256,000 of a column 0.23 and 0.18 ms, 655,000 of a collapsed one
-// 0.98 and 0.91 ms, but 1,049,000 0.61 and 0.69 ms and 8.4 M 4.14 and
-// 5.39 ms: groups compute a particle's own values once a lane, and a chip
-// filled by threads gains nothing from them.
+// Groups compute a particle's own values once a lane, and a chip filled by
+// threads gains nothing from them; how many particles fill it depends on how
+// close they lie.  Measured on a GB300 (same bits), thread against group in
+// us: the settled pile, 125,000, 443 and 337; a collapsed column with its
+// reference constants, 296,000 799 and 494, 448,000 866 and 677, 656,000 909
+// and 908, 910,000 1,046 and 1,176; one as configured, 283,000 509 and 520,
+// 633,000 676 and 900; unit masses 1.9 r apart, 200,000 120 and 125, 400,000
+// 211 and 246, 700,000 335 and 429; 2.6 r apart 100,000 47 and 47, 400,000
+// 107 and 158, 700,000 165 and 272.  8.4 M 3,905 and 5,438.
 constexpr int kSurfList = 128;
-constexpr int64_t kSurfGroupMax = 700000;
+// Merged particles have more neighbours than the lattice they came from; in
+// math mode 1 each neighbour costs more (2.6 r apart, 690,000 941 and 875).
+constexpr int64_t kSurfGroupMax = 450000, kSurfGroupMaxLong = 700000;
 
 template <int MM, int G>
 __global__ void __launch_bounds__(kSurfThreads) k_surface_group(SurfArgs a) {
@@ -373,7 +378,8 @@ gg_status surface(gg_system* S, cudaStream_t st) {
   merge_cuts(S, merge_f, a.merge_cut);
   a.ld_sum = S->g.ld_sum;
   a.ld_cnt = S->g.ld_cnt;
-  if (S->n <= kSurfGroupMax) {
+  const bool longer = S->merged_total > 0 || S->P.math_mode;
+  if (S->n <= (longer ? kSurfGroupMaxLong : kSurfGroupMax)) {
     auto kern = S->P.math_mode ? k_surface_group<1, 8> : k_surface_group<0, 8>;
     kern<<<blocks_for(S->n, kSurfThreads / 8), kSurfThreads, 0, st>>>(a);
   } else {
@@ -429,10 +435,12 @@ __global__ void __launch_bounds__(256) k_surfdist(Grid g, int n, const float4* _
 
 // The same with 8 lanes to a particle (k_surface_group's scheme): the lanes
 // look at 8 of the 27 cells at a time and share the particles of each one
-// that holds a surface particle.  Measured, thread against group: 51,000
-// particles of the box scene 0.058 and 0.034 ms, 125,000 of the settled pile
-// 0.153 and 0.079 ms, 655,000 of a collapsed column 0.30 and 0.18 ms, but
-// 1,049,000 of one at its start 0.12 and 0.15 ms.
+// that holds a surface particle.  Measured, thread against group in us: the
+// settled pile, 125,000, 154 and 79; a collapsed column, 656,000 308 and 175,
+// 1,246,000 324 and 275, 2,082,000 363 and 410; one as configured, 633,000 129
+// and 130; columns at their start, 442,000 143 and 94, 1,049,000 112 and 151;
+// unit masses 1.9 r apart, 400,000 72 and 72, 700,000 94 and 109; 2.6 r apart
+// 200,000 48 and 41, 700,000 57 and 91.
 constexpr int kDistLanes = 8;
 constexpr int64_t kDistGroupMax = 700000;
 
@@ -614,12 +622,17 @@ __global__ void __launch_bounds__(256) k_merge_scan(MergeArgs a) {
 // time; the masses within the radius are added in candidate order by one
 // lane, and of partners at equal distance the first in that order (the
 // lowest index: the particles are sorted by cell) is kept, as one thread
-// would.  All of the merge's kernels, with the scan by threads against
-// groups: box scene 0.067 and 0.056 ms, settled pile 0.129 and 0.076 ms,
-// 655,000 collapsed 0.36 and 0.23 ms, 1,049,000 0.40 and 0.34 ms, 8.4 M 1.37
-// and 1.49 ms.
+// would.  Where the merge radius covers the stencil every candidate counts,
+// and groups pay in larger systems.  All of the merge's kernels, with the scan
+// by threads against groups in us: covered, columns at their start, 1,049,000
+// 361 and 306, 2,048,000 494 and 454, 3,539,000 622 and 644, 8.4 M 1,217 and
+// 1,334, and collapsed, 656,000 358 and 230, 2,082,000 464 and 398, 4,806,000
+// 711 and 745; not covered, the settled pile, 125,000, 130 and 76, unit masses
+// 1.9 r apart, 200,000 110 and 99, 400,000 169 and 167, 1 M 232 and 264, 2 M
+// 379 and 459, 2.6 r apart 100,000 69 and 72, 500,000 135 and 157, 2 M 287 and
+// 386.
 constexpr int kMergeLanes = 8;
-constexpr int64_t kMergeGroupMax = 2000000;
+constexpr int64_t kMergeGroupMax = 500000, kMergeGroupMaxCovered = 2000000;
 
 __global__ void __launch_bounds__(256) k_merge_scan_group(MergeArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -881,8 +894,9 @@ gg_status merge_mark(gg_system* S, cudaStream_t st) {
   // particle, plus what it moved since the grid was built (the predicted
   // step and the sweeps; the ALL form stays exact either way)
   const float reach2 = 12.0f * S->grid.L * S->grid.L * 1.001f;
-  if (S->n <= kMergeGroupMax) k_merge_scan_group<<<blocks_for(S->n, 256 / kMergeLanes), 256, 0, st>>>(a);
-  else if (reach2 < a.merge_r2_cut) k_merge_scan<true><<<nb, 256, 0, st>>>(a);
+  const bool covered = reach2 < a.merge_r2_cut;
+  if (S->n <= (covered ? kMergeGroupMaxCovered : kMergeGroupMax)) k_merge_scan_group<<<blocks_for(S->n, 256 / kMergeLanes), 256, 0, st>>>(a);
+  else if (covered) k_merge_scan<true><<<nb, 256, 0, st>>>(a);
   else k_merge_scan<false><<<nb, 256, 0, st>>>(a);
   k_merge_claims<<<nb, 256, 0, st>>>(a);
   {

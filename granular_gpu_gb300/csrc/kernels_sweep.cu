@@ -1122,12 +1122,14 @@ gg_status window_table(gg_system* S, cudaStream_t st) {
   return GG_OK;
 }
 
-// Systems up to this size give every particle a group of lanes.  Measured
-// against the thread kernels with their queues left to groups, per pass:
-// 51,000 particles (10 listed each) 1.66 against 1.82 ms, 125,000 in a dense
-// pile (28 listed) 2.78 against 3.07 ms, but 144,000 loosely packed (6
-// listed) 11.3 against 9.2 ms and 643,000 (23 listed) 8.7 against 5.6 ms:
-// the line lies where a thread to a particle starts to fill the chip.
+// Systems up to this size give every particle a group of lanes.  Where threads
+// take over depends on the packing, which the host does not know; sweeps of a
+// substep by threads and by groups in us: 2.6 r apart (no neighbours) 20,000
+// 105 and 94, 60,000 108 and 163, 100,000 113 and 229; 1.9 r apart 60,000 274
+// and 246, 100,000 364 and 434; 1.5 r apart 60,000 444 and 387, 100,000 482 and
+// 540; settled piles 64,000 937 and 552, 111,000 1,338 and 898, 176,000 1,581
+// and 1,543, 262,000 2,668 and 2,786; collapsed columns 96,000 1,576 and 1,104,
+// 178,000 2,169 and 1,689, 448,000 3,140 and 3,608.
 constexpr int64_t kGroupMax = 100000;
 
 // The sweep's threads clear the increment table for its apply kernel where
