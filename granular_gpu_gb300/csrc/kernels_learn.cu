@@ -452,7 +452,8 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
 
 // One pass over the samples: loss and gradient of the mean squared error
 // between the MLP's prediction and the targets, accumulated into a.loss and
-// a.grad (fp32, one atomic add per CTA and parameter).
+// a.grad (fp32 atomic adds, per CTA one for each parameter; those of the two
+// hidden layers go four to a request).
 __global__ void __launch_bounds__(kTile, 1) k_mlp_train(const __grid_constant__ CUtensorMap tmX, MlpArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sW = smem + kTrW;

@@ -126,7 +126,7 @@ gg_status step_once(gg_system* S) {
   if (S->P.warm_start == 2 && (rc = warm_start_record(S, st)) != GG_OK) return rc;
   if (S->P.target_residual > 0.0f) {
     // residual mode: the stabilisation sweeps, then Jacobi sweeps until the
-    // largest penetration, measured before each sweep, is within the target
+    // mean penetration, measured before each sweep, is within the target
     const int stab = S->P.stab_iters;
     for (int it = 0; it < stab; ++it) {
       if ((rc = sweep(S, it, st)) != GG_OK) return rc;
