@@ -607,12 +607,13 @@ __device__ __forceinline__ float nlist_cell_bound(const SweepArgs& a, int3 q, ui
 
 // Sweeps after the first: particles whose list is still exact run it; the
 // others are queued for k_sweep_nlist_build.
-// 4 resident blocks of 256 (64 registers): substeps of the 8.4 M column 28.3 ms
-// against 28.6 with 5 (48 registers), batch of 643,000 4.40 and 4.57, warm-started
-// 144,000 4.33 and 4.66; 8 M particles falling free of each other, whose lists
-// are empty, 4.44 and 4.26.
-template <int MM>
-__global__ void __launch_bounds__(256, 4) k_sweep_nlist_keep(SweepArgs a) {
+// 4 resident blocks of 256 (64 registers) against 5 (48, and some spills): the
+// 8.4 M column 28.3 ms a substep and 28.7, warm-started 144,000 4.33 and 4.66,
+// a batch of 643,000 4.40 and 4.57.  5 in large systems under the Coulomb law
+// (kKeepWide).  8 M particles under the reference's law that fall free of each
+// other, whose lists are empty, take 4.44 ms with 4 and 4.26 with 5.
+template <int MM, int kBlocks>
+__global__ void __launch_bounds__(256, kBlocks) k_sweep_nlist_keep(SweepArgs a) {
   const Grid& g = a.g;
   const int tid = (int)pdl_wait(threadIdx.x);
   if ((MM & 4) && a.scal->res_done) return;
@@ -1132,6 +1133,12 @@ gg_status window_table(gg_system* S, cudaStream_t st) {
 // 178,000 2,169 and 1,689, 448,000 3,140 and 3,608.
 constexpr int64_t kGroupMax = 100000;
 
+// Above this size the keep kernel has 5 resident blocks under the Coulomb law,
+// with 4 and 5 in ms a substep: a batch of 7.9 M in 64 scenes 6.67 and 6.54,
+// 4.5 M particles 2.0 r apart 2.76 and 2.73, 2.6 r apart 2.00 and 1.94, 1.75 r
+// apart 3.55 and 3.55; 1.5 M 1.04 and 1.04, 0.74 and 0.73, 1.35 and 1.36.
+constexpr int64_t kKeepWide = 1500000;
+
 // The sweep's threads clear the increment table for its apply kernel where
 // that leaves each at most this many entries; a few particles in a large grid
 // leave it to a memset, which has the whole chip (and costs a launch, about
@@ -1259,7 +1266,8 @@ gg_status sweep(gg_system* S, int it, cudaStream_t st, ResidualSlot* res) {
     if (it == 0) {
       GG_CUDA(launch_chained(build, blocks_for(S->n, kBuildThreads), kBuildThreads, st, a, 0));
     } else {
-      auto keep = GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM>);
+      auto keep = S->n > kKeepWide ? GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM, (MM & 2) ? 5 : 4>)
+                                   : GG_SWEEP_KERNEL(mm, k_sweep_nlist_keep<MM, 4>);
       const int tk = S->tune.keep_threads;
       GG_CUDA(launch_chained(keep, blocks_for(S->n, tk), tk, st, a));
       const int nb = std::min(blocks_for(S->n, kBuildThreads), S->num_sms * S->tune.build_blocks_per_sm);

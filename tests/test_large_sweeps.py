@@ -11,10 +11,10 @@ from oracle import oracle as orc
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("law", [0, 1])
-@pytest.mark.parametrize("n,spacing", [(400000, 1.9), (400001, 1.4), (500000, 1.7)])
+@pytest.mark.parametrize("n,spacing,law", [(400000, 1.9, 0), (400000, 1.9, 1), (400001, 1.4, 0), (400001, 1.4, 1),
+                                           (500000, 1.7, 0), (500000, 1.7, 1), (1500001, 1.9, 1)])
 def test_laws_match_oracle(n, spacing, law):
-    r = 0.005
+    r = 0.005 if n < 1000000 else 0.004
     side = int(np.ceil(n ** (1 / 3)))
     d = workloads.box_drop(2, substeps=8, configured=law == 1)
     p = workloads.lattice((side,) * 3, spacing * r, (0.02,) * 3, 0.2 * spacing * r, 1)
