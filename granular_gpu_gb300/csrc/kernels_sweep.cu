@@ -448,8 +448,12 @@ __device__ __forceinline__ void process_entry(const SweepArgs& a, const Target& 
 // lanes of a warp walk the same cell sequence), with the candidates that
 // pass the cheap distance test listed in order and processed by all lanes
 // together afterwards.
+// 4 resident blocks of 256: it hides its loads with warps.  With the 78
+// registers that it takes unbounded (3 blocks) 2 M particles 1.9 r apart took
+// 7.34 ms of sweeps a substep, 6.08 with 64 and a few bytes spilled; 300,000
+// 1.24 and 1.02 ms, 50,000 0.438 and 0.443.
 template <int MM>
-__global__ void __launch_bounds__(kWarpThreads) k_sweep_list(SweepArgs a) {
+__global__ void __launch_bounds__(kWarpThreads, 4) k_sweep_list(SweepArgs a) {
   __shared__ int s_list[kWarpThreads / 32][kWarpList][32];
   const Grid& g = a.g;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
