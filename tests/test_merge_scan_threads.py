@@ -69,3 +69,33 @@ def test_threads_take_over_where_they_are_faster(kind, below, above):
         ms.append(best)
         g.close()
     assert ms[0] <= 1.15 * ms[1]
+
+
+@pytest.mark.parametrize("n,reach", [(450000, 0.06), (500000, 0.06), (500000, 0.02)])
+def test_one_particle_beyond_the_line_changes_nothing(n, reach):
+    """CUDA's math functions, which the oracle matches to 4 ulp only: the
+    same particles with one more far from them, which takes the system to the
+    kernels beyond the line, keep their surface flags, distances and merges."""
+    masses = np.random.default_rng(6).choice([0.5, 1.0, 2.0], n + 1).astype(np.float32)
+    masses[n] = 1.0
+    out = []
+    for more in (0, 1):
+        d = _scene(n + 1, 1.9, reach, None, 0.1)
+        length, space = np.float32(d["cell_length"]), tuple(x + 0.4 for x in d["space_size"])
+        walls, cells = workloads.box_walls(space, length)
+        p = d["particles"].copy()
+        p[n] = [x - 0.2 for x in space]  # behind all others in the cells' order
+        d.update(boundary=walls, n_boundary=len(walls), space_size=space, cell_size=tuple(cells), particles=p[:n + more],
+                 n_particles=n + more)
+        d["params"].math_mode = 0
+        g = gg.GranularSystem(**workloads.system_kwargs(d), masses=masses[:n + more], device=0)
+        fields = []
+        for _ in range(3):
+            g.step(1)
+            fields += [g.read(f)[:n] for f in (gg.FIELD_SURFACE, gg.FIELD_SURFACE_DISTANCE, gg.FIELD_REMOVE,
+                                               gg.FIELD_MERGE, gg.FIELD_MASS, gg.FIELD_POS)]
+        assert g.size() == n + more and (fields[2] != 0).any()
+        out.append(fields)
+        g.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
